@@ -561,21 +561,18 @@ __device__ __forceinline__ void kick_consts(const Consts& k, double gam, double 
   tcon = bet * xycon * (gam * gam);
 }
 
-// update_CompDom, Flagbc=1 (CompDom.f90:545-557, 614-622): eps is the
-// default-real 1.0/(Meshnum-3.0)
-__device__ __forceinline__ void compdom(Geom& g, int nx, int ny, int nz) {
-  const int mesh[3] = {nx, ny, nz};
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    double t1 = g.ptrange[2 * k], t2 = g.ptrange[2 * k + 1];
-    double eps = (double)(1.0f / ((float)mesh[k] - 3.0f));
-    double mn = t1 - eps * (t2 - t1);
-    double mx = t2 + eps * (t2 - t1);
-    g.range[2 * k] = mn;
-    g.range[2 * k + 1] = mx;
-    g.h[k] = (mx - mn) / (double)(mesh[k] - 1);
-    g.hi[k] = 1.0 / g.h[k];
-  }
+// update_CompDom, Flagbc=1 (CompDom.f90:545-557, 614-622), axis k of `mesh`
+// nodes from the particle range [t1, t2]: eps is the default-real
+// 1.0/(Meshnum-3.0)
+__device__ __forceinline__ void compdom_axis(Geom& g, int k, int mesh, double t1, double t2) {
+  const double eps = (double)(1.0f / ((float)mesh - 3.0f));
+  const double mn = t1 - eps * (t2 - t1);
+  const double mx = t2 + eps * (t2 - t1);
+  g.range[2 * k] = mn;
+  g.range[2 * k + 1] = mx;
+  const double h = (mx - mn) / (double)(mesh - 1);
+  g.h[k] = h;
+  g.hi[k] = 1.0 / h;
 }
 
 __device__ __forceinline__ bool finite6(const Particle& p) {
@@ -1206,64 +1203,94 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
   if (!s_last) return;
   __threadfence();
   // ---- last block: fixed-order reduction over blocks, then bookkeeping.
-  // Warp w reduces blocks [w*nb/nw, (w+1)*nb/nw) of every value (lane l:
-  // values l and l+32; 0..43 moments, 44..51 range), then thread v combines
-  // the warps' partials in warp order: a fixed order, and the loads of one
-  // lane are independent, so they overlap instead of chaining.
+  // It runs alone at the end of every step, so what bounds it is the latency
+  // of its loads.  The values are taken in pairs (one 16-byte load): thread
+  // (g, c) of the 22 moment pairs, or of the 4 range pairs, folds blocks g,
+  // g + groups, ... with LAST_BATCH loads in flight, then one thread per
+  // value combines the groups in order (deterministic for a grid size).  One
+  // lane per value with a dependent load per block took 31 us of every step
+  // at 296 blocks (clock counters); with this a job of 1e5 particles in the
+  // plain FP64 form went from 128 to 107 us per step, uploads included.
+  constexpr int MP = IMPZ_RAW_LEN / 2, RP = 4;  // pairs of moments and of range values
+  constexpr int RG = 8, MG = (BLOCK - RG * RP) / MP;
+  static_assert(MG * MP + RG * RP <= BLOCK && MG >= 1, "threads of the last block");
+  static_assert((MG * MP + RG * RP) * 2 <= 32 * IMPZ_MSUMS * (BLOCK / 32), "group partials");
+  constexpr int LAST_BATCH = 8;
   const int nb = vgx;
   const int row = a.fixed_step >= 0 ? a.mom_index : s;
-  const int b0 = wid * nb / nw, b1 = (wid + 1) * nb / nw;
-  for (int v = lane; v < IMPZ_RAW_LEN + 8; v += 32) {
-    const bool isrng = v >= IMPZ_RAW_LEN;
-    const int r = v - IMPZ_RAW_LEN;  // range value 0..7
-    if (!isrng && !mom) continue;
-    // identities: sums 0, maxima of |.| 0, range min +1e300 / max -1e300
-    double x = (isrng && r < 6) ? ((r & 1) ? -1e300 : 1e300) : 0.0;
-#pragma unroll 4
-    for (int b = b0; b < b1; b++) {
-      const double y = isrng ? __ldcg(a.rng_part + (size_t)b * 8 + r)
-                             : __ldcg(a.mom_part + (size_t)b * IMPZ_RAW_LEN + v);
-      if (isrng) x = (r >= 6) ? x + y : ((r & 1) ? fmax(x, y) : fmin(x, y));
-      else x = v < IMPZ_MSUMS ? x + y : fmax(x, y);
+  const int t = threadIdx.x;
+  const double cur0 = st->current;  // read now: the loads overlap the reduction
+  const long long npt0 = st->npt;
+  double2* gp = reinterpret_cast<double2*>(mtile_dyn);  // [MG][MP] then [RG][RP]
+  const bool isrng = t >= MG * MP;
+  const int ngr = isrng ? RG : MG, np = isrng ? RP : MP;
+  const int tt_ = isrng ? t - MG * MP : t;
+  const int grp = tt_ / np, cp = tt_ - grp * np;
+  if (grp < ngr && (isrng || mom)) {
+    const double2* src = reinterpret_cast<const double2*>(isrng ? a.rng_part : a.mom_part) + cp;
+    // what value pair cp holds: sums, maxima, or range minimum and maximum
+    const bool add0 = isrng ? cp == RP - 1 : 2 * cp < IMPZ_MSUMS;
+    const bool add1 = isrng ? cp == RP - 1 : 2 * cp + 1 < IMPZ_MSUMS;
+    const bool min0 = isrng && cp < RP - 1;
+    double2 x = make_double2(min0 ? 1e300 : 0.0, min0 ? -1e300 : 0.0);
+    for (int b0 = grp; b0 < nb; b0 += ngr * LAST_BATCH) {
+      double2 y[LAST_BATCH];
+#pragma unroll
+      for (int q = 0; q < LAST_BATCH; q++) {
+        const int b = b0 + q * ngr;
+        y[q] = __ldcg(src + (size_t)(b < nb ? b : grp) * np);
+      }
+#pragma unroll
+      for (int q = 0; q < LAST_BATCH; q++)
+        if (b0 + q * ngr < nb) {
+          x.x = add0 ? x.x + y[q].x : min0 ? fmin(x.x, y[q].x) : fmax(x.x, y[q].x);
+          x.y = add1 ? x.y + y[q].y : fmax(x.y, y[q].y);
+        }
     }
-    if (isrng) redr[wid][r] = x;
-    else red[wid][v] = x;
+    gp[t] = x;
   }
   __syncthreads();
-  if (mom && threadIdx.x < IMPZ_RAW_LEN) {
-    const int v = threadIdx.x;
-    double x = red[0][v];
-    for (int w = 1; w < nw; w++) x = v < IMPZ_MSUMS ? x + red[w][v] : fmax(x, red[w][v]);
-    a.mom_out[(size_t)row * IMPZ_MOMREC + v] = x;
+  const double* gd = mtile_dyn;
+  if (mom && t < IMPZ_RAW_LEN) {
+    double x = gd[t];
+#pragma unroll
+    for (int w = 1; w < MG; w++) {
+      const double y = gd[w * 2 * MP + t];
+      x = t < IMPZ_MSUMS ? x + y : fmax(x, y);
+    }
+    a.mom_out[(size_t)row * IMPZ_MOMREC + t] = x;
   }
-  if (threadIdx.x < 8) {
-    const int v = threadIdx.x;
-    double x = redr[0][v];
-    for (int w = 1; w < nw; w++) {
-      const double y = redr[w][v];
+  if (t >= BLOCK - 8) {  // another warp than the moments'
+    const int v = t - (BLOCK - 8);
+    const double* rd = gd + 2 * MG * MP + v;
+    double x = rd[0];
+#pragma unroll
+    for (int w = 1; w < RG; w++) {
+      const double y = rd[w * 2 * RP];
       x = (v >= 6) ? x + y : ((v & 1) ? fmax(x, y) : fmin(x, y));
     }
     fin[v] = x;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (t < 3 && rng) {  // update_CompDom, one axis per thread
+    st->geom.ptrange[2 * t] = fin[2 * t];
+    st->geom.ptrange[2 * t + 1] = fin[2 * t + 1];
+    compdom_axis(st->geom, t, t == 0 ? nx : t == 1 ? ny : nz, fin[2 * t], fin[2 * t + 1]);
+  }
+  if (t == 32) {
     const long long kept = (long long)fin[7];
     if (mom) {
       double* m = a.mom_out + (size_t)row * IMPZ_MOMREC;
-      m[44] = (double)st->npt;
+      m[44] = (double)npt0;
       m[45] = (double)kept;
-      m[46] = st->current;
+      m[46] = cur0;
       m[47] = 0.0;
     }
     st->nlocal = kept;
     if (rng) {
-      Geom ng;
-      for (int d = 0; d < 6; d++) ng.ptrange[d] = fin[d];
-      compdom(ng, nx, ny, nz);
-      st->geom = ng;
       const long long nptot = (long long)fin[6];
       // conv1st: Current = Current*nptot/Npt; Npt = nptot
-      st->current = st->current * (double)nptot / (double)st->npt;
+      st->current = cur0 * (double)nptot / (double)npt0;
       st->npt = nptot;
       st->nlive = nptot;
     }
