@@ -29,7 +29,8 @@ NVCC_COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
 UNITS = [
     ("impz_particle_exact.cu", ["--fmad=false"]),
     ("impz_particle_fast.cu", []),
-    ("impz_poisson.cu", ["--fmad=false"]),
+    ("impz_poisson_f32.cu", ["--fmad=false"]),
+    ("impz_poisson_f64.cu", ["--fmad=false"]),
     ("impz_capi.cu", []),
     ("impz_serve.cu", []),
     ("impz_static.cu", ["--fmad=false"]),

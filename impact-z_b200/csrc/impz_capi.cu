@@ -337,7 +337,7 @@ size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 struct Layout {
   size_t pbuf[2][6], ids[2], spc[2], sptab, rho, counts, cursor, bsum, spec, F, ghat, phi,
       efield;
-  size_t tw[3], tw64[3], st, dfine, mom_fine, mom_part, rng_part, flag;
+  size_t tw[3], st, dfine, mom_fine, mom_part, rng_part, flag;
   size_t total;
   int nscan;
 };
@@ -375,11 +375,8 @@ Layout plan_layout(long long n, int nx, int ny, int nz, int form, int flags) {
   L.ghat = take(noct * esz);
   L.phi = take(G * esz);
   L.efield = take(4 * G * esz);
-  const int half[3] = {nx, ny, nz};  // a length-2m transform keeps m twiddles
-  for (int d = 0; d < 3; d++) {
-    L.tw64[d] = take((size_t)half[d] * sizeof(double2));
-    L.tw[d] = take((size_t)half[d] * 2 * esz);
-  }
+  const int half[3] = {nx, ny, nz};  // a length-2m transform keeps up to 2m twiddles
+  for (int d = 0; d < 3; d++) L.tw[d] = take((size_t)half[d] * 2 * 2 * esz);
   L.st = take(sizeof(DevState));
   L.dfine = take(2 * sizeof(StepParams));
   L.mom_fine = take(IMPZ_MOMREC * sizeof(double));
@@ -453,7 +450,6 @@ struct impz_bunch_s {
   void* phi = nullptr;
   void* efield = nullptr;
   void* tw[3] = {nullptr, nullptr, nullptr};
-  double2* tw64[3] = {nullptr, nullptr, nullptr};
   DevState* st = nullptr;
   StepParams* dsteps = nullptr;
   StepParams* dfine = nullptr;  // 2-entry table of the per-call surface
@@ -462,7 +458,6 @@ struct impz_bunch_s {
   double* mom_out = nullptr;
   double* mom_fine = nullptr;
   int grid_adv = 0, grid_dep = 0;
-  int ztile = 0;  // z lines per block of the z convolution (0: the largest that fits)
   BendState bend;
   int stage = ST_IDLE;
   double sc_gam = 0, sc_rad = 0;
@@ -546,12 +541,10 @@ PoissonBuffers poisson_of(impz_bunch_t b) {
   pb.spec = b->spec; pb.F = b->F; pb.ghat = b->ghat;
   pb.phi = b->phi; pb.efield = b->efield;
   pb.twx = b->tw[0]; pb.twy = b->tw[1]; pb.twz = b->tw[2];
-  pb.tw64x = b->tw64[0]; pb.tw64y = b->tw64[1]; pb.tw64z = b->tw64[2];
   pb.st = b->st;
   const bool wake = b->run_wake;
   pb.wake = wake ? b->wk_field : nullptr;
   pb.wake_line = wake ? b->wk_line : nullptr;
-  pb.ztile = b->ztile;
   return pb;
 }
 
@@ -954,16 +947,6 @@ int upload_pts(impz_bunch_t b, const double* pts, long long n) {
   return upload_order(b, n);
 }
 
-template <typename C>
-void fill_tw(std::vector<C>& v, int n) {
-  v.resize(n / 2 > 0 ? n / 2 : 1);
-  for (int k = 0; k < n / 2; k++) {
-    const double a = -2.0 * M_PI * (double)k / (double)n;
-    v[k].x = (decltype(v[k].x))std::cos(a);
-    v[k].y = (decltype(v[k].y))std::sin(a);
-  }
-}
-
 void free_bunch(impz_bunch_t b) {
   if (!b) return;
   cudaSetDevice(b->device);
@@ -1035,9 +1018,6 @@ int impz_bunch_create(const double* pts, long long n, double current, double mas
   if (!(mass > 0) || !(freq > 0) || charge == 0.0) return IMPZ_ERR_ARG;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return IMPZ_ERR_NODEVICE;
-  if (!(form == IMPZ_FORM_FP32CONV ? poisson_fits<float>(nx, ny, nz)
-                                   : poisson_fits<double>(nx, ny, nz)))
-    return IMPZ_ERR_UNSUPPORTED;  // a z line of the doubled grid exceeds shared memory
   impz_bunch_t b = new impz_bunch_s();
   cudaGetDevice(&b->device);
   b->form = form;
@@ -1104,10 +1084,7 @@ int impz_bunch_create(const double* pts, long long n, double current, double mas
   b->ghat = at(L.ghat);
   b->phi = at(L.phi);
   b->efield = at(L.efield);
-  for (int d = 0; d < 3; d++) {
-    b->tw64[d] = (double2*)at(L.tw64[d]);
-    b->tw[d] = at(L.tw[d]);
-  }
+  for (int d = 0; d < 3; d++) b->tw[d] = at(L.tw[d]);
   b->st = (DevState*)at(L.st);
   b->dfine = (StepParams*)at(L.dfine);
   b->mom_fine = (double*)at(L.mom_fine);
@@ -1120,16 +1097,11 @@ int impz_bunch_create(const double* pts, long long n, double current, double mas
   ALLOC(cudaMemsetAsync(b->counts, 0, (G + 1) * sizeof(int), b->stream));
   const int lens[3] = {2 * nx, 2 * ny, 2 * nz};
   for (int d = 0; d < 3; d++) {
-    std::vector<double2> t64;
-    fill_tw(t64, lens[d]);
-    ALLOC(cudaMemcpy(b->tw64[d], t64.data(), t64.size() * sizeof(double2), cudaMemcpyHostToDevice));
-    if (b->f32()) {
-      std::vector<float2> t32;
-      fill_tw(t32, lens[d]);
-      ALLOC(cudaMemcpy(b->tw[d], t32.data(), t32.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    } else {
-      ALLOC(cudaMemcpy(b->tw[d], t64.data(), t64.size() * sizeof(double2), cudaMemcpyHostToDevice));
-    }
+    std::vector<double2> t(lens[d]);
+    const int m = b->f32() ? fft_twiddles<float>(ilog2i(lens[d]), t.data())
+                           : fft_twiddles<double>(ilog2i(lens[d]), t.data());
+    ALLOC(cudaMemcpy(b->tw[d], t.data(), (size_t)m * (b->f32() ? sizeof(float2) : sizeof(double2)),
+                     cudaMemcpyHostToDevice));
   }
   b->grid_adv = (int)std::min<long long>((n + IMPZ_ADV_BLOCK - 1) / IMPZ_ADV_BLOCK,
                                          (long long)(b->f32() ? fast::max_blocks_advance(true)
@@ -1997,11 +1969,7 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
   std::vector<BatchGroup> groups;
   for (int k = 0; k < nb; k++) {
     const impz_bunch_t b = bs[order[k]];
-    PoissonBuffers pb = poisson_of(b);
-    PoissonMember& m = mem[k];
-    m.rho = pb.rho; m.qscale = pb.qscale; m.spec = pb.spec; m.ghat = pb.ghat; m.phi = pb.phi;
-    m.efield = pb.efield; m.twx = pb.twx; m.twy = pb.twy; m.twz = pb.twz; m.F = pb.F;
-    m.st = pb.st;
+    mem[k] = poisson_member(poisson_of(b));
     if (groups.empty() || groups.back().nx != b->nx || groups.back().ny != b->ny ||
         groups.back().nz != b->nz)
       groups.push_back(BatchGroup{b->nx, b->ny, b->nz, k, 0});
@@ -2193,11 +2161,7 @@ static int packed_step(impz_bunch_t* bs, int nb, cudaStream_t s, cudaStream_t s2
   std::vector<BatchGroup> groups;
   for (int k = 0; k < ns; k++) {
     const impz_bunch_t b = sc_b[order[k]];
-    const PoissonBuffers pb = poisson_of(b);
-    PoissonMember& m = pm[k];
-    m.rho = pb.rho; m.qscale = pb.qscale; m.spec = pb.spec; m.ghat = pb.ghat; m.phi = pb.phi;
-    m.efield = pb.efield; m.twx = pb.twx; m.twy = pb.twy; m.twz = pb.twz; m.F = pb.F;
-    m.st = pb.st;
+    pm[k] = poisson_member(poisson_of(b));
     if (groups.empty() || groups.back().nx != b->nx || groups.back().ny != b->ny ||
         groups.back().nz != b->nz)
       groups.push_back(BatchGroup{b->nx, b->ny, b->nz, k, 0});
@@ -2582,15 +2546,13 @@ int impz_autotune(impz_bunch_t b, int nsteps, double out[4]) {
     return IMPZ_OK;
   };
   if (!r) {
-    std::vector<int> dc, ac, zc;
+    std::vector<int> dc, ac;
     for (int v : {dep0, dep0 / 2, 2 * sms, 4 * sms, 8 * sms})
       if (v >= 1 && v <= std::min(dep0, dep_need)) dc.push_back(v);
     for (int v : {adv0, adv0 / 2, sms, 2 * sms, 3 * sms})
       if (v >= 1 && v <= std::min(std::min(adv0, adv_need), kMaxAdvGrid)) ac.push_back(v);
-    for (int v : {8, 4, 2}) zc.push_back(v);
     r = sweep(&b->grid_dep, dc);
     if (!r) r = sweep(&b->grid_adv, ac);
-    if (!r) r = sweep(&b->ztile, zc);
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -2601,7 +2563,7 @@ int impz_autotune(impz_bunch_t b, int nsteps, double out[4]) {
   if (r2) return r2;
   out[0] = b->grid_dep;
   out[1] = b->grid_adv;
-  out[2] = b->ztile;
+  out[2] = 0.0;  // the z convolution has one shape per length
   out[3] = best;
   return IMPZ_OK;
 }

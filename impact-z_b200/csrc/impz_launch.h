@@ -76,25 +76,32 @@ IMPZ_DECLARE_PARTICLE_LAUNCHERS(fast)
 // Poisson solve (T = double for the FP64 form, float for the FP32 form)
 struct PoissonBuffers {
   int nx, ny, nz;
-  unsigned long long* rho;  // int64 charge, cleared by the forward pass
+  unsigned long long* rho;  // int64 charge, cleared by the field kernel
   double qscale;            // grid value of one fixed-point quantum
   void* spec;               // (nx+1)*2ny*nz complex T
   double* F;                // (nx+2)(ny+2)(nz+2) IGF corners
   void* ghat;               // (nx+1)(ny+1)(nz+1) T
   void* phi;                // nx*ny*nz T
   void* efield;             // 4*nx*ny*nz T
-  const void* twx;          // twiddles of length 2nx, 2ny, 2nz in T
+  const void* twx;          // twiddles of length 2nx, 2ny, 2nz in T (fft_twiddles)
   const void* twy;
   const void* twz;
-  const double2* tw64x;     // FP64 twiddles for the DCT of G
-  const double2* tw64y;
-  const double2* tw64z;
   DevState* st;
   const double* wake;       // per-plane {dEx, dEy, dEz}[nz] added to E, or null
   unsigned long long* wake_line;  // the wake's [3][nz] line sums, cleared with the charge
-  int ztile;                // z lines per block of the z convolution (0: the largest that fits)
 };
 
+// the part of the buffers the solve of one bunch among several needs
+inline PoissonMember poisson_member(const PoissonBuffers& b) {
+  PoissonMember m;
+  m.rho = b.rho; m.qscale = b.qscale; m.spec = b.spec; m.ghat = b.ghat; m.phi = b.phi;
+  m.efield = b.efield; m.twx = b.twx; m.twy = b.twy; m.twz = b.twz; m.F = b.F; m.st = b.st;
+  return m;
+}
+
+// twiddles of a transform of 2^logn points (complex T, at most 2^logn entries)
+template <typename T>
+int fft_twiddles(int logn, void* out);
 template <typename T>
 cudaError_t launch_green(const PoissonBuffers& b, cudaStream_t s);
 template <typename T>
@@ -111,13 +118,6 @@ cudaError_t launch_efield(const PoissonBuffers& b, cudaStream_t s);
 template <typename T>
 cudaError_t launch_green_group(int nx, int ny, int nz, const PoissonMember* mem, int nmem,
                                cudaStream_t s);
-template <typename T>
-cudaError_t launch_conv_group(int nx, int ny, int nz, const PoissonMember* mem, int nmem,
-                              cudaStream_t s);
-template <typename T>
-cudaError_t launch_efield_group(int nx, int ny, int nz, const PoissonMember* mem, int nmem,
-                                cudaStream_t s);
-// launch_conv_group split where G-hat is first needed
 template <typename T>
 cudaError_t launch_conv_group_forward(int nx, int ny, int nz, const PoissonMember* mem, int nmem,
                                       cudaStream_t s);

@@ -5,431 +5,381 @@
 // integrated Green's function G, then kick1's finite-difference field
 // (src/Appl/BeamBunch.f90:1784-2005).  Any correct FFT reproduces the
 // reference's FFTPACK convolution to rounding, so the transforms here are the
-// project's own shared-memory radix-2 kernels laid out for the doubled grid:
+// project's own register FFTs (impz_fft.cuh) laid out for the doubled grid:
 //
 //   xy-forward  one block per z plane: int64 charge -> real, R2C along x
 //               (two real rows packed into one complex FFT of length 2Nx),
 //               C2C along y (length 2Ny, upper half zero), spectrum plane out
-//   z-convolve  one block per (ky, tile of kx): C2C along z (length 2Nz,
-//               upper half zero), times the real even G-hat, inverse C2C,
-//               only the Nz planes the crop needs are written back
+//   z-convolve  a few lines per block: C2C along z (length 2Nz, upper half
+//               zero), times the real even G-hat, inverse C2C, only the Nz
+//               planes the crop needs are written back
 //   xy-inverse  one block per z plane < Nz: inverse C2C along y, C2R along x,
 //               potential plane out (only Nx x Ny of the doubled grid)
+//
+// After the x transform the kx = 0 and kx = Nx rows are real, so they travel
+// through the y transform as one complex line: a plane has Nx lines, a power
+// of two, and the pair is separated (joined) where the spectrum is stored
+// (loaded).
 //
 // G is even in every direction, so its transform is real and is computed as
 // three DCT-I passes over the octant (Nx+1)(Ny+1)(Nz+1) (two lines packed
 // into one complex FFT: even real sequences have real transforms).  The
 // 1/(n1 n2 n3) inverse normalisation of Field.f90:321-323 is folded into G-hat.
 //
-// Spectrum layout in HBM: S[z][ky][kx], kx fastest, (Nx+1) x 2Ny x Nz complex.
-// Forward passes use decimation in frequency (natural in, bit-reversed out)
-// and inverse passes decimation in time (bit-reversed in, natural out), so no
-// pass ever permutes data explicitly.
+// Layouts in HBM.  The z convolution is the pass with the long lines, so the
+// spectrum is stored for it: the lines are grouped, 2T to a group (T values
+// of the line index q at ky and the same T at 2Ny - ky), and a group's
+// points lie together, z by z, S[group][z][side][T]: a block reads and
+// writes one contiguous piece, and the xy passes touch whole 32-byte sectors
+// (T = 4 FP32 values).  T is 4, and less where the lines are so long that
+// fewer fit a block (zt_log).  Line q = row * Nx + kx for kx < Nx, and
+// Ny * Nx + row for kx = Nx, with row = ky (side 0) or 2Ny - ky (side 1; row
+// 0 holds ky = 0 and ky = Ny).  G-hat holds T lines together in the same
+// way, ((q / T) (Nz+1) + kz) T + q mod T with q = ky Nx + kx, then the kx =
+// Nx lines, and the last line (ky = Ny, kx = Nx) alone.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "impz_common.h"
 #include "impz_device.cuh"
+#include "impz_fft.cuh"
 
 namespace impz {
-
-template <typename T> struct Cplx;
-template <> struct Cplx<double> { typedef double2 type; };
-template <> struct Cplx<float> { typedef float2 type; };
-
-template <typename C>
-__device__ __forceinline__ C cadd(C a, C b) { C r; r.x = a.x + b.x; r.y = a.y + b.y; return r; }
-template <typename C>
-__device__ __forceinline__ C csub(C a, C b) { C r; r.x = a.x - b.x; r.y = a.y - b.y; return r; }
-template <typename C>
-__device__ __forceinline__ C cmul(C a, C b) {
-  C r; r.x = a.x * b.x - a.y * b.y; r.y = a.x * b.y + a.y * b.x; return r;
-}
-
-__device__ __forceinline__ int bitrev(int v, int logn) {
-  return (int)(__brev((unsigned)v) >> (32 - logn));
-}
-
-// Lines in shared memory keep one spare slot after every eight elements:
-// element j of a line sits at sw(j).  The butterfly groups read eight
-// elements a fixed spacing apart, and at the small spans consecutive
-// threads start eight elements apart, which without the spare slots would
-// put 16 threads of a warp on the same banks.
-__device__ __forceinline__ int sw(int j) { return j + (j >> 3); }
-// line pitch (in elements) for lines of n >= 8 elements: odd, past sw(n-1)
-__host__ __device__ constexpr int line_pitch(int n) { return n + n / 8 + 1; }
-
-// Radix-2 butterflies over `nlines` lines in shared memory; element j of
-// line l sits at buf[l*lstride + sw(j)].  tw[k] = exp(-2 pi i k / n), k < n/2.
-// DIF: natural order in, bit-reversed out.  DIT: bit-reversed in, natural out.
-// Up to three consecutive radix-2 stages act on the 2^NS elements spaced by
-// the narrowest span, so each thread runs them in registers (one barrier and
-// one shared-memory round trip per NS stages); the butterflies, twiddles and output order are those of plain
-// radix-2.  Within a group, a stage with pair distance se uses only se
-// distinct twiddles: element e pairs at position k + (e mod se) q, so the se
-// twiddles are loaded once per stage and shared by its butterflies.
-template <typename C>
-__device__ __forceinline__ C twid(const C* tw, int idx, int sign) {
-  C w = tw[idx];
-  if (sign > 0) w.y = -w.y;
-  return w;
-}
-
-// stages with half-spans 2^lh, 2^(lh-1), .., 2^(lh-NS+1) (DIF)
-template <typename C, int NS>
-__device__ __forceinline__ void dif_group(C* L, int o, int logn, int lh, int k, int sign,
-                                          const C* tw) {
-  constexpr int E = 1 << NS;
-  const int q = 1 << (lh - NS + 1);  // spacing of the E elements
-  C v[E];
-#pragma unroll
-  for (int e = 0; e < E; e++) v[e] = L[sw(o + k + e * q)];
-#pragma unroll
-  for (int m = 0; m < NS; m++) {
-    const int se = E >> (m + 1);      // pair distance; 2^(lh-m) = se * q
-    const int tsh = logn - 1 - (lh - m);
-    C w[E / 2];
-#pragma unroll
-    for (int j = 0; j < se; j++) w[j] = twid(tw, (k + j * q) << tsh, sign);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      if (e & se) continue;
-      const C u = v[e], t = v[e + se];
-      v[e] = cadd(u, t);
-      v[e + se] = cmul(csub(u, t), w[e & (se - 1)]);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < E; e++) L[sw(o + k + e * q)] = v[e];
-}
-
-// stages with half-spans 2^lh, .., 2^(lh+NS-1) (DIT)
-template <typename C, int NS>
-__device__ __forceinline__ void dit_group(C* L, int o, int logn, int lh, int k, int sign,
-                                          const C* tw) {
-  constexpr int E = 1 << NS;
-  const int q = 1 << lh;
-  C v[E];
-#pragma unroll
-  for (int e = 0; e < E; e++) v[e] = L[sw(o + k + e * q)];
-#pragma unroll
-  for (int m = 0; m < NS; m++) {
-    const int se = 1 << m;            // pair distance; 2^(lh+m) = se * q
-    const int tsh = logn - 1 - (lh + m);
-    C w[E / 2];
-#pragma unroll
-    for (int j = 0; j < se; j++) w[j] = twid(tw, (k + j * q) << tsh, sign);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      if (e & se) continue;
-      const C u = v[e], t = cmul(v[e + se], w[e & (se - 1)]);
-      v[e] = cadd(u, t);
-      v[e + se] = csub(u, t);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < E; e++) L[sw(o + k + e * q)] = v[e];
-}
-
-// widest group: three stages (four for FP32 lines spent more registers than
-// the fewer rounds saved)
-#ifndef IMPZ_FFT_NS_F32
-#define IMPZ_FFT_NS_F32 3
-#endif
-template <typename C>
-struct MaxStages { static constexpr int value = sizeof(C) == 8 ? IMPZ_FFT_NS_F32 : 3; };
-
-template <typename C>
-__device__ void fft_dif(C* buf, int logn, int nlines, int lstride, int sign, const C* tw) {
-  constexpr int MS = MaxStages<C>::value;
-  int lh = logn - 1;
-  while (lh >= 0) {
-    const int ns = lh + 1 >= MS ? MS : lh + 1;
-    const int lper = lh - ns + 1;            // log2 of the groups per block
-    const int lngl = logn - ns;              // log2 of the groups per line
-    const int total = nlines << lngl;
-    for (int b = threadIdx.x; b < total; b += blockDim.x) {
-      const int l = b >> lngl, r = b & ((1 << lngl) - 1);
-      const int o = (r >> lper) << (lh + 1), k = r & ((1 << lper) - 1);
-      C* Lp = buf + l * lstride;
-      if (MS >= 4 && ns == 4) dif_group<C, (MS >= 4 ? 4 : 1)>(Lp, o, logn, lh, k, sign, tw);
-      else if (ns == 3) dif_group<C, 3>(Lp, o, logn, lh, k, sign, tw);
-      else if (ns == 2) dif_group<C, 2>(Lp, o, logn, lh, k, sign, tw);
-      else dif_group<C, 1>(Lp, o, logn, lh, k, sign, tw);
-    }
-    __syncthreads();
-    lh -= ns;
-  }
-}
-
-template <typename C>
-__device__ void fft_dit(C* buf, int logn, int nlines, int lstride, int sign, const C* tw) {
-  constexpr int MS = MaxStages<C>::value;
-  int lh = 0;
-  while (lh < logn) {
-    const int ns = (logn - lh) >= MS ? MS : logn - lh;
-    const int lngl = logn - ns;
-    const int total = nlines << lngl;
-    for (int b = threadIdx.x; b < total; b += blockDim.x) {
-      const int l = b >> lngl, r = b & ((1 << lngl) - 1);
-      const int o = (r >> lh) << (lh + ns), k = r & ((1 << lh) - 1);
-      C* Lp = buf + l * lstride;
-      if (MS >= 4 && ns == 4) dit_group<C, (MS >= 4 ? 4 : 1)>(Lp, o, logn, lh, k, sign, tw);
-      else if (ns == 3) dit_group<C, 3>(Lp, o, logn, lh, k, sign, tw);
-      else if (ns == 2) dit_group<C, 2>(Lp, o, logn, lh, k, sign, tw);
-      else dit_group<C, 1>(Lp, o, logn, lh, k, sign, tw);
-    }
-    __syncthreads();
-    lh += ns;
-  }
-}
-
-// copies n/2 twiddles into shared memory (whole block, no barrier)
-template <typename C>
-__device__ __forceinline__ void stage_tw(C* dst, const C* __restrict__ src, int n) {
-  for (int e = threadIdx.x; e < n / 2; e += blockDim.x) dst[e] = src[e];
-}
 
 struct PoissonDims {
   int nx, ny, nz;
   int lx, ly, lz;  // log2 of the doubled lengths 2nx, 2ny, 2nz
 };
 
-// ---------------------------------------------------------------------
-// xy-forward: PARTS blocks per z plane k < nz (one by default: splitting a
-// plane measured slower at 64x64).  Each block transforms all the plane's
-// rows along x and then unpacks, transforms along y and stores its own share
-// of the nx+1 kx lines.  The charge is cleared later, by k_efield (not by
-// stores interleaved with the transform's loads).
-// smem: Z[ny/2][2nx] (packed row pairs) and Tm[own kx][2ny] (y lines).
-template <typename T, int PARTS>
-__device__ __forceinline__ void fft_xy_fwd_body(const PoissonDims& d,
-                                                const unsigned long long* __restrict__ rho,
-                                                double qscale, typename Cplx<T>::type* __restrict__ S,
-                                                const typename Cplx<T>::type* __restrict__ twx,
-                                                const typename Cplx<T>::type* __restrict__ twy,
-                                                const int bx, const int by) {
+// log2 of T, the lines of one side of a group, for z transforms of 2^lz points
+template <typename T>
+__host__ __device__ constexpr int zt_log(int lz) {
+  return sizeof(T) == 4 ? (lz <= 9 ? 2 : lz == 10 ? 1 : 0) : (lz <= 8 ? 2 : lz == 9 ? 1 : 0);
+}
+
+// element index of spectrum line (ky, kx) at plane z
+__device__ __forceinline__ size_t spec_index(const PoissonDims& d, int lt, int ky, int kx, int z) {
+  const int n2 = 2 * d.ny;
+  const int side = ky >= d.ny ? 1 : 0;
+  const int row = ky < d.ny ? ky : ky == d.ny ? 0 : n2 - ky;
+  const int q = kx < d.nx ? row * d.nx + kx : d.ny * d.nx + row;
+  return (((size_t)(q >> lt) * d.nz + z) << (lt + 1)) + (side << lt) + (q & ((1 << lt) - 1));
+}
+
+// first element and spacing along kz of line (ky, kx) of G-hat (ky <= ny, kx <= nx)
+__device__ __forceinline__ size_t ghat_line(int nx, int ny, int nz, int lt, int ky, int kx,
+                                            int& spacing) {
+  const int q = kx < nx ? ky * nx + kx : (ny + 1) * nx + ky;
+  spacing = (kx == nx && ky == ny) ? 1 : 1 << lt;
+  return (((size_t)(q >> lt) * (nz + 1)) << lt) + (q & ((1 << lt) - 1));
+}
+
+__host__ __device__ constexpr int round_to(int v, int m) { return (v + m - 1) / m * m; }
+
+// The xy kernels' shape: lines of the x transform (row pairs) and of the y
+// transform, each rounded to whole warps (the spare lines are scratch), the
+// pitches of their lines, and the block.  The pitches put the transposing
+// reads between the two transforms on different banks: 2 mod 16 eight-byte
+// slots (FP32), odd sixteen-byte slots (FP64).
+template <typename T, int LX, int LY>
+struct XyShape {
+  typedef Fft<T, LX> FX;
+  typedef Fft<T, LY> FY;
   typedef typename Cplx<T>::type C;
+  static constexpr int nx = 1 << (LX - 1), ny = 1 << (LY - 1), hy = ny / 2;
+  static constexpr int TA = round_to(hy * FX::TPL, 32), TB = round_to(nx * FY::TPL, 32);
+  static constexpr int LA = TA / FX::TPL, LB = TB / FY::TPL;
+  static constexpr int extra = sizeof(T) == 4 ? 2 : 1;
+  static constexpr int XP = FX::LEN + extra, YP = FY::LEN + extra;
+  static constexpr int NT = TA > TB ? TA : TB;
+  // the x and y lines are never needed at the same time
+  static constexpr size_t smem = sizeof(C) * (size_t)(LA * XP > LB * YP ? LA * XP : LB * YP);
+};
+
+// The bunch a block works for: the *_group launches give the members of a
+// group of one grid size in device memory (blockIdx.y = member), a solo
+// launch passes its own by value.  Copied, not referred to: a reference that
+// may point to either was compiled into reads of the wrong one.
+__device__ __forceinline__ PoissonMember member_of(const PoissonMember& one,
+                                                   const PoissonMember* __restrict__ many) {
+  PoissonMember m = one;
+  if (many) m = many[blockIdx.y];
+  return m;
+}
+
+// ---------------------------------------------------------------------
+// xy-forward: one block per z plane.  Bound by latency (128 planes on 148
+// SMs at 64x64x128): every thread holds its part of one line, so a plane
+// takes two register transforms, three block barriers and one exchange of
+// the plane in between.
+template <typename T, int LX, int LY>
+__device__ __forceinline__ void fft_xy_fwd_body(const PoissonDims& d, const PoissonMember& mm) {
+  typedef XyShape<T, LX, LY> X;
+  typedef typename X::FX FX;
+  typedef typename X::FY FY;
+  typedef typename Cplx<T>::type C;
+  constexpr int nx = X::nx, ny = X::ny, hy = X::hy, n1 = 2 * nx, n2 = 2 * ny;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* sm = reinterpret_cast<C*>(smem_raw);
+  const int tid = threadIdx.x, z = blockIdx.x;
   griddep_wait();
-  const int nx = d.nx, ny = d.ny, n1 = 2 * nx, n2 = 2 * ny, w = nx + 1;
-  const int zp = line_pitch(n1), tp = line_pitch(n2);  // x-line and y-line pitches
-  const int hy = ny / 2;
-  const int part = bx, k = by;
-  const int kx_lo = w * part / PARTS, nown = w * (part + 1) / PARTS - kx_lo;
-  C* Z = reinterpret_cast<C*>(smem_raw);
-  C* Tm = Z + hy * zp;
-  C* twxs = Tm + ((w + PARTS - 1) / PARTS) * tp;
-  C* twys = twxs + n1 / 2;
-  stage_tw(twxs, twx, n1);
-  stage_tw(twys, twy, n2);
-  const size_t plane = (size_t)nx * ny * k;
-  // load two real rows per complex line, natural order, zero padded
-  for (int e = threadIdx.x; e < hy * n1; e += blockDim.x) {
-    const int l = e >> d.lx, j = e & (n1 - 1);
-    C z;
-    z.x = 0; z.y = 0;
-    if (j < nx) {
-      const size_t ia = plane + (size_t)l * nx + j, ib = plane + (size_t)(l + hy) * nx + j;
-      z.x = (T)((double)(long long)rho[ia] * qscale);
-      z.y = (T)((double)(long long)rho[ib] * qscale);
-    }
-    Z[l * zp + sw(j)] = z;
-  }
-  __syncthreads();
-  fft_dif<C>(Z, d.lx, hy, zp, -1, twxs);
-  // unpack: row a = (Z(k)+conj(Z(n1-k)))/2, row b = (Z(k)-conj(Z(n1-k)))/(2i),
-  // own kx, into y lines Tm[kx - kx_lo][y] (natural y, zero padded to 2ny)
-  for (int e = threadIdx.x; e < nown * n2; e += blockDim.x) {
-    const int kl = e >> d.ly, y = e & (n2 - 1);
-    const int kx = kx_lo + kl;
-    C v;
-    v.x = 0; v.y = 0;
-    if (y < ny) {
-      const int l = y < hy ? y : y - hy;
-      const C* L = Z + l * zp;
-      const C zk = L[sw(bitrev(kx, d.lx))];
-      const C zm = L[sw(bitrev((n1 - kx) & (n1 - 1), d.lx))];
-      if (y < hy) {
-        v.x = (T)0.5 * (zk.x + zm.x);
-        v.y = (T)0.5 * (zk.y - zm.y);
-      } else {
-        v.x = (T)0.5 * (zk.y + zm.y);
-        v.y = (T)0.5 * (zm.x - zk.x);
+  const unsigned long long* rho = mm.rho + (size_t)nx * ny * z;
+  if (tid < X::TA) {  // rows l and l + hy as one complex line
+    const int l = tid / FX::TPL, j = tid % FX::TPL;
+    C v[FX::E];
+#pragma unroll
+    for (int e = 0; e < FX::E / 2; e++) {
+      const int x = j + FX::TPL * e;
+      v[e].x = 0;
+      v[e].y = 0;
+      if (l < hy) {
+        v[e].x = (T)((double)(long long)rho[l * nx + x] * mm.qscale);
+        v[e].y = (T)((double)(long long)rho[(l + hy) * nx + x] * mm.qscale);
       }
     }
-    Tm[kl * tp + sw(y)] = v;
+    C* L = sm + l * X::XP;
+    FX::template run<-1, true>(v, j, L, (const C*)mm.twx, WarpSync());
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < FX::E; e++) L[FX::pad(j + FX::TPL * e)] = v[e];
   }
   __syncthreads();
-  fft_dif<C>(Tm, d.ly, nown, tp, -1, twys);
-  // store S[k][ky][kx] for the own kx, (ky, kl) walked with a carry
-  C* Sk = S + (size_t)k * n2 * w + kx_lo;
-  {
-    const int dky = blockDim.x / nown, dkl = blockDim.x - dky * nown;
-    int ky = threadIdx.x / nown, kl = threadIdx.x - ky * nown;
-    for (int e = threadIdx.x; e < nown * n2; e += blockDim.x) {
-      Sk[(size_t)ky * w + kl] = Tm[kl * tp + sw(bitrev(ky, d.ly))];
-      kl += dkl;
-      ky += dky;
-      if (kl >= nown) { kl -= nown; ky++; }
+  // unpack: row a = (Z(k)+conj(Z(n1-k)))/2, row b = (Z(k)-conj(Z(n1-k)))/(2i);
+  // at kx = 0 both rows' kx = 0 and kx = nx values (real) as one complex line
+  const int kx = tid / FY::TPL, j = tid % FY::TPL;
+  C v[FY::E];
+  if (tid < X::TB) {
+#pragma unroll
+    for (int e = 0; e < FY::E / 4; e++) {
+      C a, b;
+      a.x = a.y = b.x = b.y = 0;
+      if (kx < nx) {
+        const C* L = sm + (j + FY::TPL * e) * X::XP;
+        const C zk = L[FX::pad(kx)];
+        const C zm = L[FX::pad(kx ? n1 - kx : nx)];
+        if (kx) {
+          a.x = (T)0.5 * (zk.x + zm.x);
+          a.y = (T)0.5 * (zk.y - zm.y);
+          b.x = (T)0.5 * (zk.y + zm.y);
+          b.y = (T)0.5 * (zm.x - zk.x);
+        } else {
+          a.x = zk.x; a.y = zm.x;
+          b.x = zk.y; b.y = zm.y;
+        }
+      }
+      v[e] = a;
+      v[e + FY::E / 4] = b;
+    }
+  }
+  __syncthreads();
+  if (tid >= X::TB) return;
+  C* L = sm + kx * X::YP;
+  FY::template run<-1, true>(v, j, L, (const C*)mm.twy, WarpSync());
+  C* S = (C*)mm.spec;
+  const int lt = zt_log<T>(d.lz);
+  if (kx > 0 && kx < nx) {
+#pragma unroll
+    for (int e = 0; e < FY::E; e++) S[spec_index(d, lt, j + FY::TPL * e, kx, z)] = v[e];
+  }
+  if (tid < 32) {  // the warp of the packed line: separate its two real rows
+    __syncwarp();
+    if (kx == 0) {
+#pragma unroll
+      for (int e = 0; e < FY::E; e++) L[FY::pad(j + FY::TPL * e)] = v[e];
+    }
+    __syncwarp();
+    if (kx == 0) {
+#pragma unroll
+      for (int e = 0; e < FY::E; e++) {
+        const int ky = j + FY::TPL * e;
+        const C m = L[FY::pad((n2 - ky) & (n2 - 1))];
+        C a, b;
+        a.x = (T)0.5 * (v[e].x + m.x);
+        a.y = (T)0.5 * (v[e].y - m.y);
+        b.x = (T)0.5 * (v[e].y + m.y);
+        b.y = (T)0.5 * (m.x - v[e].x);
+        S[spec_index(d, lt, ky, 0, z)] = a;
+        S[spec_index(d, lt, ky, nx, z)] = b;
+      }
     }
   }
 }
 
-template <typename T, int PARTS>
-__global__ void k_fft_xy_fwd(PoissonDims d, const unsigned long long* __restrict__ rho,
-                             double qscale, typename Cplx<T>::type* __restrict__ S,
-                             const typename Cplx<T>::type* __restrict__ twx,
-                             const typename Cplx<T>::type* __restrict__ twy) {
-  fft_xy_fwd_body<T, PARTS>(d, rho, qscale, S, twx, twy, blockIdx.x, blockIdx.y);
+template <typename T, int LX, int LY>
+__global__ void __launch_bounds__((XyShape<T, LX, LY>::NT))
+    k_fft_xy_fwd(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many) {
+  fft_xy_fwd_body<T, LX, LY>(d, member_of(one, many));
 }
 
-// the same for every bunch of a group of one grid size: blockIdx.z = member
-template <typename T, int PARTS>
-__global__ void k_fft_xy_fwd_group(PoissonDims d, const PoissonMember* __restrict__ mem) {
-  typedef typename Cplx<T>::type C;
-  const PoissonMember& m = mem[blockIdx.z];
-  fft_xy_fwd_body<T, PARTS>(d, m.rho, m.qscale, (C*)m.spec, (const C*)m.twx, (const C*)m.twy,
-                            blockIdx.x, blockIdx.y);
-}
-
-// z-convolve: block = (tile of TKX kx values, one ky).
-template <typename T, int TKX>
-__device__ __forceinline__ void fft_z_conv_body(const PoissonDims& d,
-                                                typename Cplx<T>::type* __restrict__ S,
-                                                const T* __restrict__ ghat,
-                                                const typename Cplx<T>::type* __restrict__ twz,
-                                                const int bx, const int by) {
-  typedef typename Cplx<T>::type C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  griddep_wait();
-  const int nx = d.nx, ny = d.ny, nz = d.nz, n2 = 2 * ny, n3 = 2 * nz;
-  const int lp = line_pitch(n3);
-  C* L = reinterpret_cast<C*>(smem_raw);
-  C* twzs = L + TKX * lp;
-  stage_tw(twzs, twz, n3);
-  const int kx0 = bx * TKX;
-  const int ky = by;
-  const int ntk = min(TKX, nx + 1 - kx0);
-  const size_t pstride = (size_t)n2 * (nx + 1);  // one z plane of S
-  C* base = S + (size_t)ky * (nx + 1) + kx0;
-  for (int e = threadIdx.x; e < TKX * n3; e += blockDim.x) {
-    const int z = e / TKX, t = e - z * TKX;
-    C v;
-    v.x = 0; v.y = 0;
-    if (z < nz && t < ntk) v = base[(size_t)z * pstride + t];
-    L[t * lp + sw(z)] = v;
-  }
-  __syncthreads();
-  fft_dif<C>(L, d.lz, TKX, lp, -1, twzs);
-  // multiply by G-hat (bit-reversed positions); G-hat octant [kz'][ky'][kx]
-  const int kyp = ky <= ny ? ky : n2 - ky;
-  const size_t gy = (size_t)(nx + 1), gz = (size_t)(nx + 1) * (ny + 1);
-  for (int e = threadIdx.x; e < TKX * n3; e += blockDim.x) {
-    const int t = e >> d.lz, pos = e & (n3 - 1);
-    if (t >= ntk) continue;
-    const int kz = bitrev(pos, d.lz);
-    const int kzp = kz <= nz ? kz : n3 - kz;
-    const T gv = ghat[(size_t)kzp * gz + (size_t)kyp * gy + kx0 + t];
-    C& v = L[t * lp + sw(pos)];
-    v.x *= gv;
-    v.y *= gv;
-  }
-  __syncthreads();
-  fft_dit<C>(L, d.lz, TKX, lp, +1, twzs);
-  for (int e = threadIdx.x; e < TKX * nz; e += blockDim.x) {
-    const int z = e / TKX, t = e - z * TKX;
-    if (t < ntk) base[(size_t)z * pstride + t] = L[t * lp + sw(z)];
-  }
-}
-
-template <typename T, int TKX>
-__global__ void k_fft_z_conv(PoissonDims d, typename Cplx<T>::type* __restrict__ S,
-                             const T* __restrict__ ghat,
-                             const typename Cplx<T>::type* __restrict__ twz) {
-  fft_z_conv_body<T, TKX>(d, S, ghat, twz, blockIdx.x, blockIdx.y);
-}
-
-template <typename T, int TKX>
-__global__ void k_fft_z_conv_group(PoissonDims d, const PoissonMember* __restrict__ mem) {
-  typedef typename Cplx<T>::type C;
-  const PoissonMember& m = mem[blockIdx.z];
-  fft_z_conv_body<T, TKX>(d, (C*)m.spec, (const T*)m.ghat, (const C*)m.twz, blockIdx.x,
-                          blockIdx.y);
-}
-
+// ---------------------------------------------------------------------
 // xy-inverse: one block per z plane k < nz; phi out (nx, ny, nz) real.
-template <typename T>
-__device__ __forceinline__ void fft_xy_inv_body(const PoissonDims& d,
-                                                const typename Cplx<T>::type* __restrict__ S,
-                                                T* __restrict__ phi,
-                                                const typename Cplx<T>::type* __restrict__ twx,
-                                                const typename Cplx<T>::type* __restrict__ twy,
-                                                const int bx) {
+template <typename T, int LX, int LY>
+__device__ __forceinline__ void fft_xy_inv_body(const PoissonDims& d, const PoissonMember& mm) {
+  typedef XyShape<T, LX, LY> X;
+  typedef typename X::FX FX;
+  typedef typename X::FY FY;
   typedef typename Cplx<T>::type C;
+  constexpr int nx = X::nx, ny = X::ny, hy = X::hy, n1 = 2 * nx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* sm = reinterpret_cast<C*>(smem_raw);
+  const int tid = threadIdx.x, z = blockIdx.x;
+  const int lt = zt_log<T>(d.lz);
   griddep_wait();
-  const int nx = d.nx, ny = d.ny, n1 = 2 * nx, n2 = 2 * ny;
-  const int zp = line_pitch(n1), tp = line_pitch(n2);
-  const int hy = ny / 2;
-  C* Z = reinterpret_cast<C*>(smem_raw);
-  C* Tm = Z + hy * zp;
-  C* twxs = Tm + (nx + 1) * tp;
-  C* twys = twxs + n1 / 2;
-  stage_tw(twxs, twx, n1);
-  stage_tw(twys, twy, n2);
-  const int k = bx;
-  const C* Sk = S + (size_t)k * n2 * (nx + 1);
-  // y lines in bit-reversed order for the DIT inverse
-  {
-    const int w = nx + 1, dky = blockDim.x / w, dkx = blockDim.x - dky * w;
-    int ky = threadIdx.x / w, kx = threadIdx.x - ky * w;
-    for (int e = threadIdx.x; e < w * n2; e += blockDim.x) {
-      Tm[kx * tp + sw(bitrev(ky, d.ly))] = Sk[e];
-      kx += dkx;
-      ky += dky;
-      if (kx >= w) { kx -= w; ky++; }
+  if (tid < X::TB) {
+    const int kx = tid / FY::TPL, j = tid % FY::TPL;
+    const C* S = (const C*)mm.spec;
+    C v[FY::E];
+#pragma unroll
+    for (int e = 0; e < FY::E; e++) {
+      v[e].x = 0;
+      v[e].y = 0;
+      if (kx < nx) v[e] = S[spec_index(d, lt, j + FY::TPL * e, kx, z)];
+      if (kx == 0) {  // the kx = 0 and kx = nx rows as one complex line
+        const C b = S[spec_index(d, lt, j + FY::TPL * e, nx, z)];
+        v[e].x = v[e].x - b.y;
+        v[e].y = v[e].y + b.x;
+      }
+    }
+    C* L = sm + kx * X::YP;
+    FY::template run<1, false>(v, j, L, (const C*)mm.twy, WarpSync());
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < FY::E / 2; e++) L[FY::pad(j + FY::TPL * e)] = v[e];
+  }
+  __syncthreads();
+  // C2R along x for row pairs (l, l + hy): Z(kx) = Xa(kx) + i Xb(kx), with
+  // X(n1-kx) = conj(X(kx))
+  const int l = tid / FX::TPL, j = tid % FX::TPL;
+  C v[FX::E];
+  if (tid < X::TA) {
+#pragma unroll
+    for (int e = 0; e < FX::E; e++) {
+      const int kk = j + FX::TPL * e;
+      v[e].x = 0;
+      v[e].y = 0;
+      if (l < hy) {
+        const C* L = sm + ((kk == nx ? 0 : kk < nx ? kk : n1 - kk) * X::YP);
+        C xa = L[FY::pad(l)], xb = L[FY::pad(l + hy)];
+        if (kk == 0) { xa.y = 0; xb.y = 0; }
+        if (kk == nx) { xa.x = xa.y; xb.x = xb.y; xa.y = 0; xb.y = 0; }
+        if (kk > nx) { xa.y = -xa.y; xb.y = -xb.y; }
+        v[e].x = xa.x - xb.y;
+        v[e].y = xa.y + xb.x;
+      }
     }
   }
   __syncthreads();
-  fft_dit<C>(Tm, d.ly, nx + 1, tp, +1, twys);
-  // C2R along x for row pairs (y, y+ny/2), y < ny/2: Z(kx) = Xa(kx) + i Xb(kx),
-  // with X(n1-kx) = conj(X(kx)); placed bit-reversed for the DIT inverse
-  for (int e = threadIdx.x; e < hy * n1; e += blockDim.x) {
-    const int l = e >> d.lx, kk = e & (n1 - 1);
-    const int kxs = kk <= nx ? kk : n1 - kk;
-    C xa = Tm[kxs * tp + sw(l)], xb = Tm[kxs * tp + sw(l + hy)];
-    if (kk > nx) { xa.y = -xa.y; xb.y = -xb.y; }
-    C z;
-    z.x = xa.x - xb.y;
-    z.y = xa.y + xb.x;
-    Z[l * zp + sw(bitrev(kk, d.lx))] = z;
-  }
-  __syncthreads();
-  fft_dit<C>(Z, d.lx, hy, zp, +1, twxs);
-  T* ph = phi + (size_t)nx * ny * k;
-  for (int e = threadIdx.x; e < nx * ny; e += blockDim.x) {
-    const int y = e >> (d.lx - 1), x = e & (nx - 1);
-    const C v = Z[(y < hy ? y : y - hy) * zp + sw(x)];
-    ph[e] = y < hy ? v.x : v.y;
+  if (tid >= X::TA) return;
+  FX::template run<1, false>(v, j, sm + l * X::XP, (const C*)mm.twx, WarpSync());
+  if (l >= hy) return;
+  T* ph = (T*)mm.phi + (size_t)nx * ny * z;
+#pragma unroll
+  for (int e = 0; e < FX::E / 2; e++) {
+    const int x = j + FX::TPL * e;
+    ph[l * nx + x] = v[e].x;
+    ph[(l + hy) * nx + x] = v[e].y;
   }
 }
 
-template <typename T>
-__global__ void k_fft_xy_inv(PoissonDims d, const typename Cplx<T>::type* __restrict__ S,
-                             T* __restrict__ phi,
-                             const typename Cplx<T>::type* __restrict__ twx,
-                             const typename Cplx<T>::type* __restrict__ twy) {
-  fft_xy_inv_body<T>(d, S, phi, twx, twy, blockIdx.x);
+template <typename T, int LX, int LY>
+__global__ void __launch_bounds__((XyShape<T, LX, LY>::NT))
+    k_fft_xy_inv(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many) {
+  fft_xy_inv_body<T, LX, LY>(d, member_of(one, many));
 }
 
-template <typename T>
-__global__ void k_fft_xy_inv_group(PoissonDims d, const PoissonMember* __restrict__ mem) {
+// ---------------------------------------------------------------------
+// The z kernels' shape.  PAR lines are in work at once, thread (j, line)
+// with the lines fastest: the spectrum's group and the threads of a warp run
+// along the same contiguous piece.  The pitch puts the lines of a half
+// (quarter) warp on different banks.
+template <typename T, int LZ, int PAR>
+struct ZShape {
+  typedef Fft<T, LZ> F;
+  static constexpr int slots = 128 / (int)(2 * sizeof(T));  // of one shared-memory wavefront
+  static constexpr int want = PAR < slots ? slots / PAR : 1;
+  static constexpr int P0 = F::LEN;
+  static constexpr int pitch = P0 + (want + slots - P0 % slots) % slots;
+  static constexpr int NT = PAR * F::TPL;
+  static constexpr size_t smem = sizeof(typename Cplx<T>::type) * (size_t)PAR * pitch;
+};
+
+// lines of the z convolution in work at once: a whole group, several groups
+// where the lines are short, one line where a block of 1024 threads holds
+// no more (8192 points in FP64)
+template <typename T, int LZ>
+struct ZConv {
+  typedef Fft<T, LZ> F;
+  static constexpr int lt = zt_log<T>(LZ), NL = 2 << lt;
+  static constexpr int GPB = NL * F::TPL >= 128 ? 1 : 128 / (NL * F::TPL);  // groups per block
+  static constexpr int PAR = NL * F::TPL > 1024 ? 1024 / F::TPL : NL * GPB;
+  static constexpr int ROUNDS = NL * GPB / PAR;
+  typedef ZShape<T, LZ, PAR> Z;
+};
+
+template <typename T, int LZ>
+__device__ __forceinline__ void fft_z_conv_body(const PoissonDims& d, const PoissonMember& mm) {
+  typedef ZConv<T, LZ> Q;
+  typedef typename Q::F F;
   typedef typename Cplx<T>::type C;
-  const PoissonMember& m = mem[blockIdx.y];
-  fft_xy_inv_body<T>(d, (const C*)m.spec, (T*)m.phi, (const C*)m.twx, (const C*)m.twy,
-                     blockIdx.x);
+  constexpr int lt = Q::lt, NL = Q::NL, nz = F::N / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* sm = reinterpret_cast<C*>(smem_raw);
+  const int nx = d.nx, ny = d.ny;
+  const int ngroups = (ny * nx + ny) >> lt;
+  const int j = (int)threadIdx.x / Q::PAR, p = (int)threadIdx.x % Q::PAR;
+  griddep_wait();
+#pragma unroll 1
+  for (int r = 0; r < Q::ROUNDS; r++) {
+    const int slot = r * Q::PAR + p;  // of the block's NL * GPB lines
+    const int g = blockIdx.x * Q::GPB + slot / NL, l = slot % NL;
+    const bool live = g < ngroups;
+    C* S = (C*)mm.spec + (size_t)(live ? g : 0) * nz * NL + l;
+    // the line's place, and G-hat's line for it
+    const int q = (g << lt) + (l & ((1 << lt) - 1));
+    int row, kx;
+    if (q < nx * ny) { row = q >> (d.lx - 1); kx = q & (nx - 1); }
+    else { row = q - nx * ny; kx = nx; }
+    const int kyp = (l >> lt) && row == 0 ? ny : row;
+    int gs = 1;
+    const T* G = (const T*)mm.ghat + (live ? ghat_line(nx, ny, nz, lt, kyp, kx, gs) : 0);
+    C v[F::E];
+    T gv[F::E];
+#pragma unroll
+    for (int e = 0; e < F::E / 2; e++) {
+      const int z = j + F::TPL * e;
+      v[e].x = 0;
+      v[e].y = 0;
+      if (live) v[e] = S[(size_t)z * NL];
+    }
+#pragma unroll
+    for (int e = 0; e < F::E; e++) {
+      const int kz = j + F::TPL * e;
+      gv[e] = 0;
+      if (live) gv[e] = __ldg(G + (size_t)(e < F::E / 2 ? kz : F::N - kz) * gs);
+    }
+    C* L = sm + p * Q::Z::pitch;
+    F::template run<-1, true>(v, j, L, (const C*)mm.twz, BlockSync());
+#pragma unroll
+    for (int e = 0; e < F::E; e++) {
+      v[e].x *= gv[e];
+      v[e].y *= gv[e];
+    }
+    F::template run<1, false>(v, j, L, (const C*)mm.twz, BlockSync());
+    if (live) {
+#pragma unroll
+      for (int e = 0; e < F::E / 2; e++) S[(size_t)(j + F::TPL * e) * NL] = v[e];
+    }
+  }
+}
+
+// The three passes of a step took 70 us at 64x64x128 in FP32 as radix-2^3
+// groups in shared memory and take 35 so (FP64 97 and 56); at 64x64x2048,
+// where the spectrum (136 MB) no longer fits L2, 1498 and 501.
+template <typename T, int LZ>
+__global__ void __launch_bounds__((ZConv<T, LZ>::Z::NT))
+    k_fft_z_conv(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many) {
+  fft_z_conv_body<T, LZ>(d, member_of(one, many));
 }
 
 // ---------------------------------------------------------------------
@@ -461,12 +411,9 @@ __device__ __forceinline__ void igf_corners_body(int nx, int ny, int nz, const D
   }
 }
 
-__global__ void k_igf_corners(int nx, int ny, int nz, const DevState* st, double* F) {
-  igf_corners_body(nx, ny, nz, st, F);
-}
-
-__global__ void k_igf_corners_group(int nx, int ny, int nz, const PoissonMember* __restrict__ mem) {
-  const PoissonMember& m = mem[blockIdx.y];
+static __global__ void k_igf_corners(int nx, int ny, int nz, PoissonMember one,
+                              const PoissonMember* __restrict__ many) {
+  const PoissonMember m = member_of(one, many);
   igf_corners_body(nx, ny, nz, m.st, m.F);
 }
 
@@ -476,33 +423,41 @@ __global__ void k_igf_corners_group(int nx, int ny, int nz, const PoissonMember*
 // (rows, then columns, two lines per complex FFT of length 2n), written to
 // plane k of G-hat; the z pass follows.  One pass over the corners and one
 // write of the plane instead of a difference kernel and two strided DCT
-// passes through global memory.  lx, ly: log2(2 nx), log2(2 ny).
-// smem: the line pairs of the longer transform, the twiddles of both, and
-// the plane P[(ny+1)][(nx+1)] (T).
-template <typename T>
-__device__ __forceinline__ void green_xy_body(int nx, int ny, int lx, int ly,
-                                              const double* __restrict__ F, T* __restrict__ ghat,
-                                              const typename Cplx<T>::type* __restrict__ twx,
-                                              const typename Cplx<T>::type* __restrict__ twy,
-                                              const int k) {
+// passes through global memory.
+template <typename T, int LX, int LY>
+struct GreenShape {
+  typedef Fft<T, LX> FX;
+  typedef Fft<T, LY> FY;
   typedef typename Cplx<T>::type C;
+  static constexpr int nx = 1 << (LX - 1), ny = 1 << (LY - 1), gx = nx + 1, gy = ny + 1;
+  static constexpr int npx = (gy + 1) / 2;  // row pairs (t, t + npx) for the x transform
+  static constexpr int npy = (gx + 1) / 2;  // column pairs for the y transform
+  static constexpr int TA = round_to(npx * FX::TPL, 32), TB = round_to(npy * FY::TPL, 32);
+  static constexpr int LA = TA / FX::TPL, LB = TB / FY::TPL;
+  static constexpr int NF = TA > TB ? TA : TB;
+  static constexpr int NT = NF < 512 && gx * gy > 1024 ? 512 : NF;  // for the difference pass
+  static constexpr size_t lines = LA * FX::LEN > LB * FY::LEN ? LA * FX::LEN : LB * FY::LEN;
+  static constexpr size_t smem = sizeof(C) * lines + sizeof(T) * (size_t)gx * gy;
+};
+
+template <typename T, int LX, int LY>
+__device__ __forceinline__ void green_xy_body(const PoissonDims& d, const PoissonMember& mm) {
+  typedef GreenShape<T, LX, LY> X;
+  typedef typename X::FX FX;
+  typedef typename X::FY FY;
+  typedef typename Cplx<T>::type C;
+  constexpr int nx = X::nx, ny = X::ny, gx = X::gx, gy = X::gy, ax = nx + 2, ay = ny + 2;
+  constexpr int npx = X::npx, npy = X::npy;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int gx = nx + 1, gy = ny + 1, ax = nx + 2, ay = ny + 2;
-  const int lpx = line_pitch(2 * nx), lpy = line_pitch(2 * ny);
-  const int npx = (gy + 1) / 2;  // row pairs (j, j + npx) for the x transform
-  const int npy = (gx + 1) / 2;  // column pairs (i, i + npy) for the y transform
-  C* L = reinterpret_cast<C*>(smem_raw);
-  C* twxs = L + max(npx * lpx, npy * lpy);
-  C* twys = twxs + nx;
-  T* P = reinterpret_cast<T*>(twys + ny);
-  stage_tw(twxs, twx, 2 * nx);
-  stage_tw(twys, twy, 2 * ny);
-  const double* F0 = F + (size_t)ax * ay * k;  // corner planes k and k + 1
+  C* sm = reinterpret_cast<C*>(smem_raw);
+  T* P = reinterpret_cast<T*>(sm + X::lines);
+  const int tid = threadIdx.x, k = blockIdx.x;
+  const double* F0 = mm.F + (size_t)ax * ay * k;  // corner planes k and k + 1
   const double* F1 = F0 + (size_t)ax * ay;
 #pragma unroll 4
-  for (int e = threadIdx.x; e < gx * gy; e += blockDim.x) {
+  for (int e = tid; e < gx * gy; e += X::NT) {
     const int j = e / gx, i = e - j * gx;
-#define IMPZ_F(p, a, b) __ldg(p + (a) + (size_t)ax * (b))
+#define IMPZ_F(p, a, b) __ldg(p + (a) + ax * (b))
     const double v = IMPZ_F(F1, i + 1, j + 1) - IMPZ_F(F1, i, j + 1) - IMPZ_F(F1, i + 1, j) +
                      IMPZ_F(F1, i, j) - IMPZ_F(F0, i + 1, j + 1) + IMPZ_F(F0, i, j + 1) +
                      IMPZ_F(F0, i + 1, j) - IMPZ_F(F0, i, j);
@@ -510,126 +465,109 @@ __device__ __forceinline__ void green_xy_body(int nx, int ny, int lx, int ly,
     P[e] = (T)v;
   }
   __syncthreads();
-  // along x: row t with row t + npx (real and imaginary parts)
-  for (int e = threadIdx.x; e < npx * 2 * nx; e += blockDim.x) {
-    const int m = e / npx, t = e - m * npx;
-    const int mm = m <= nx ? m : 2 * nx - m;
-    C v;
-    v.x = P[t * gx + mm];
-    v.y = t + npx < gy ? P[(t + npx) * gx + mm] : (T)0;
-    L[t * lpx + sw(m)] = v;
+  if (tid < X::TA) {  // along x: row t with row t + npx (real and imaginary parts)
+    const int t = tid / FX::TPL, j = tid % FX::TPL;
+    C v[FX::E];
+#pragma unroll
+    for (int e = 0; e < FX::E; e++) {
+      const int m = j + FX::TPL * e, m1 = m <= nx ? m : 2 * nx - m;
+      v[e].x = t < npx ? P[t * gx + m1] : (T)0;
+      v[e].y = t + npx < gy ? P[(t + npx) * gx + m1] : (T)0;
+    }
+    FX::template run<-1, false>(v, j, sm + t * FX::LEN, (const C*)mm.twx, WarpSync());
+#pragma unroll
+    for (int e = 0; e < FX::E; e++) {
+      const int m = j + FX::TPL * e;
+      if (m > nx) continue;
+      if (t < npx) P[t * gx + m] = v[e].x;
+      if (t + npx < gy) P[(t + npx) * gx + m] = v[e].y;
+    }
   }
   __syncthreads();
-  fft_dif<C>(L, lx, npx, lpx, -1, twxs);
-  for (int e = threadIdx.x; e < npx * gx; e += blockDim.x) {
-    const int m = e / npx, t = e - m * npx;
-    const C v = L[t * lpx + sw(bitrev(m, lx))];
-    P[t * gx + m] = v.x;
-    if (t + npx < gy) P[(t + npx) * gx + m] = v.y;
-  }
-  __syncthreads();
-  // along y: column t with column t + npy
-  for (int e = threadIdx.x; e < npy * 2 * ny; e += blockDim.x) {
-    const int m = e / npy, t = e - m * npy;
-    const int mm = m <= ny ? m : 2 * ny - m;
-    C v;
-    v.x = P[mm * gx + t];
-    v.y = t + npy < gx ? P[mm * gx + t + npy] : (T)0;
-    L[t * lpy + sw(m)] = v;
-  }
-  __syncthreads();
-  fft_dif<C>(L, ly, npy, lpy, -1, twys);
-  T* out = ghat + (size_t)gx * gy * k;
-  for (int e = threadIdx.x; e < npy * gy; e += blockDim.x) {
-    const int m = e / npy, t = e - m * npy;
-    const C v = L[t * lpy + sw(bitrev(m, ly))];
-    out[(size_t)m * gx + t] = v.x;
-    if (t + npy < gx) out[(size_t)m * gx + t + npy] = v.y;
+  if (tid >= X::TB) return;
+  {  // along y: column t with column t + npy
+    const int t = tid / FY::TPL, j = tid % FY::TPL;
+    const int lt = zt_log<T>(d.lz);
+    C v[FY::E];
+#pragma unroll
+    for (int e = 0; e < FY::E; e++) {
+      const int m = j + FY::TPL * e, m1 = m <= ny ? m : 2 * ny - m;
+      v[e].x = t < npy ? P[m1 * gx + t] : (T)0;
+      v[e].y = t + npy < gx ? P[m1 * gx + t + npy] : (T)0;
+    }
+    FY::template run<-1, false>(v, j, sm + t * FY::LEN, (const C*)mm.twy, WarpSync());
+    T* out = (T*)mm.ghat;
+#pragma unroll
+    for (int e = 0; e < FY::E; e++) {
+      const int m = j + FY::TPL * e;
+      if (m > ny) continue;
+      int gs;
+      if (t < npy) {
+        const size_t b = ghat_line(nx, ny, d.nz, lt, m, t, gs);
+        out[b + (size_t)k * gs] = v[e].x;
+      }
+      if (t + npy < gx) {
+        const size_t b = ghat_line(nx, ny, d.nz, lt, m, t + npy, gs);
+        out[b + (size_t)k * gs] = v[e].y;
+      }
+    }
   }
 }
 
-#ifndef IMPZ_GREEN_THREADS
-#define IMPZ_GREEN_THREADS 512
-#endif
-template <typename T>
-__global__ void __launch_bounds__(IMPZ_GREEN_THREADS)
-    k_green_xy(int nx, int ny, int lx, int ly, const double* __restrict__ F, T* __restrict__ ghat,
-               const typename Cplx<T>::type* __restrict__ twx,
-               const typename Cplx<T>::type* __restrict__ twy) {
-  green_xy_body<T>(nx, ny, lx, ly, F, ghat, twx, twy, blockIdx.x);
+template <typename T, int LX, int LY>
+__global__ void __launch_bounds__((GreenShape<T, LX, LY>::NT))
+    k_green_xy(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many) {
+  green_xy_body<T, LX, LY>(d, member_of(one, many));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(IMPZ_GREEN_THREADS)
-    k_green_xy_group(int nx, int ny, int lx, int ly, const PoissonMember* __restrict__ mem) {
+// DCT-I (transform of the even extension) along z of G-hat's lines, in
+// place, times `scale`: lines 2p and 2p + 1 (neighbours in storage) as the
+// real and imaginary parts of one complex FFT of length 2nz.
+template <typename T, int LZ>
+struct ZDct {
+  typedef Fft<T, LZ> F;
+  static constexpr int PAR = F::TPL >= 128 ? 1 : 128 / F::TPL > 16 ? 16 : 128 / F::TPL;
+  typedef ZShape<T, LZ, PAR> Z;
+  static constexpr int NT = round_to(Z::NT, 32);
+};
+
+template <typename T, int LZ>
+__device__ __forceinline__ void dct_z_body(const PoissonDims& d, const PoissonMember& mm,
+                                           T scale) {
+  typedef ZDct<T, LZ> Q;
+  typedef typename Q::F F;
   typedef typename Cplx<T>::type C;
-  const PoissonMember& m = mem[blockIdx.y];
-  green_xy_body<T>(nx, ny, lx, ly, m.F, (T*)m.ghat, (const C*)m.twx, (const C*)m.twy,
-                   blockIdx.x);
-}
-
-// DCT-I (transform of the even extension) along one axis of the octant.
-// Lines have n+1 points spaced by `es`; TL lines spaced by `ls` are handled
-// by one block (consecutive inner lines for coalescing), outer lines are
-// spaced by `os`.  Pairs of lines share one complex FFT of length 2n in the
-// compute type CT.  Reads `in` (TI), writes `out` (TO, may alias `in`: each
-// block owns its lines) times `scale`.
-template <typename TI, typename TO, typename CT, int TL>
-__device__ __forceinline__ void dct1_body(const TI* in, TO* out, int logn, long long es,
-                                          long long ls, int ninner, long long os, double scale,
-                                          const typename Cplx<CT>::type* __restrict__ tw,
-                                          const int bx, const int by) {
-  typedef typename Cplx<CT>::type C;
+  constexpr int lt = zt_log<T>(LZ), nz = F::N / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* L = reinterpret_cast<C*>(smem_raw);
-  const int n = 1 << (logn - 1);  // octant points - 1
-  const int n2 = 2 * n;
-  const int lp = line_pitch(n2);
-  C* tws = L + (TL / 2) * lp;
-  stage_tw(tws, tw, n2);
-  const int l0 = bx * TL;
-  const int nl = min(TL, ninner - l0);
-  const long long off = (long long)by * os + (long long)l0 * ls;
-  const TI* ib = in + off;
-  TO* ob = out + off;
-  // pair line t with line t + TL/2 (real and imaginary parts)
-  const int np = TL / 2;
-  for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
-    const int m = e / np, t = e - m * np;  // t fastest for coalescing
-    const int mm = m <= n ? m : n2 - m;
-    C v;
-    v.x = t < nl ? (CT)ib[(long long)t * ls + mm * es] : (CT)0;
-    v.y = t + np < nl ? (CT)ib[(long long)(t + np) * ls + mm * es] : (CT)0;
-    L[t * lp + sw(m)] = v;
+  C* sm = reinterpret_cast<C*>(smem_raw);
+  const int nlines = (d.nx + 1) * (d.ny + 1);
+  const int j = (int)threadIdx.x / Q::PAR, p = (int)threadIdx.x % Q::PAR;
+  const int qa = 2 * (blockIdx.x * Q::PAR + p), qb = qa + 1;
+  const bool la = qa < nlines && j < F::TPL, lb = qb < nlines && j < F::TPL;
+  const int sa = qa == nlines - 1 ? 1 : 1 << lt, sb = qb == nlines - 1 ? 1 : 1 << lt;
+  T* A = (T*)mm.ghat + (la ? (((size_t)(qa >> lt) * (nz + 1)) << lt) + (qa & ((1 << lt) - 1)) : 0);
+  T* B = (T*)mm.ghat + (lb ? (((size_t)(qb >> lt) * (nz + 1)) << lt) + (qb & ((1 << lt) - 1)) : 0);
+  C v[F::E];
+#pragma unroll
+  for (int e = 0; e < F::E; e++) {
+    const int m = j + F::TPL * e, m1 = m <= nz ? m : F::N - m;
+    v[e].x = la ? A[(size_t)m1 * sa] : (T)0;
+    v[e].y = lb ? B[(size_t)m1 * sb] : (T)0;
   }
-  __syncthreads();
-  fft_dif<C>(L, logn, np, lp, -1, tws);
-  for (int e = threadIdx.x; e < np * (n + 1); e += blockDim.x) {
-    const int m = e / np, t = e - m * np;
-    const C v = L[t * lp + sw(bitrev(m, logn))];
-    if (t < nl) ob[(long long)t * ls + m * es] = (TO)((double)v.x * scale);
-    if (t + np < nl) ob[(long long)(t + np) * ls + m * es] = (TO)((double)v.y * scale);
+  F::template run<-1, false>(v, j, sm + p * Q::Z::pitch, (const C*)mm.twz, BlockSync());
+#pragma unroll
+  for (int e = 0; e < F::E; e++) {
+    const int m = j + F::TPL * e;
+    if (m > nz) continue;
+    if (la) A[(size_t)m * sa] = v[e].x * scale;
+    if (lb) B[(size_t)m * sb] = v[e].y * scale;
   }
 }
 
-template <typename TI, typename TO, typename CT, int TL>
-__global__ void k_dct1(const TI* in, TO* out, int logn, long long es, long long ls, int ninner,
-                       long long os, double scale,
-                       const typename Cplx<CT>::type* __restrict__ tw) {
-  dct1_body<TI, TO, CT, TL>(in, out, logn, es, ls, ninner, os, scale, tw, blockIdx.x, blockIdx.y);
-}
-
-// pass `axis` (0: x from the FP64 octant Gt into G-hat, 1: y, 2: z in place
-// on G-hat) for every member of a group: blockIdx.z = member
-template <typename TI, typename TO, typename CT, int TL>
-__global__ void k_dct1_group(int axis, int logn, long long es, long long ls, int ninner,
-                             long long os, double scale, const PoissonMember* __restrict__ mem) {
-  typedef typename Cplx<CT>::type C;
-  const PoissonMember& m = mem[blockIdx.z];
-  const TI* in = (const TI*)m.ghat;  // x and y are done by k_green_xy_group
-  const C* tw = (const C*)(axis == 0 ? m.twx : axis == 1 ? m.twy : m.twz);
-  dct1_body<TI, TO, CT, TL>(in, (TO*)m.ghat, logn, es, ls, ninner, os, scale, tw, blockIdx.x,
-                            blockIdx.y);
+template <typename T, int LZ>
+__global__ void __launch_bounds__((ZDct<T, LZ>::NT))
+    k_dct_z(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many, T scale) {
+  dct_z_body<T, LZ>(d, member_of(one, many), scale);
 }
 
 // ---------------------------------------------------------------------
@@ -639,62 +577,47 @@ __global__ void k_dct1_group(int axis, int logn, long long es, long long ls, int
 // done) for the next deposit.  With a wake (read-in or CSR), adds its
 // per-plane field wake = {dEx, dEy, dEz}[nz] to every node of the plane
 // (kick1wake, BeamBunch.f90:5015-5033) and clears the wake's line sums.
+// One node per thread, its place by shifts (the sides are powers of two; the
+// 64-bit divisions of an earlier form kept the kernel at half of the issue
+// rate), one 16-byte store (two in FP64).
+__device__ __forceinline__ void store_field(float* E, int e, float x, float y, float z) {
+  reinterpret_cast<float4*>(E)[e] = make_float4(x, y, z, 0.f);
+}
+__device__ __forceinline__ void store_field(double* E, int e, double x, double y, double z) {
+  reinterpret_cast<double2*>(E)[2 * e] = make_double2(x, y);
+  reinterpret_cast<double2*>(E)[2 * e + 1] = make_double2(z, 0.0);
+}
+
 template <typename T>
-__device__ __forceinline__ void efield_body(int nx, int ny, int nz, const T* __restrict__ phi,
-                                            const DevState* st, T* __restrict__ E,
-                                            unsigned long long* __restrict__ rho,
-                                            const double* __restrict__ wake,
-                                            unsigned long long* __restrict__ wake_line) {
+__global__ void __launch_bounds__(256)
+    k_efield(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many,
+             const double* __restrict__ wake, unsigned long long* __restrict__ wake_line) {
+  const PoissonMember mm = member_of(one, many);
   griddep_wait();
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int e = blockIdx.x * 256 + threadIdx.x;
   if (wake_line)
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 3 * nz; e += gridDim.x * blockDim.x)
-      wake_line[e] = 0ull;
-  const long long G = (long long)nx * ny * nz;
-  const T hxi = (T)st->geom.hi[0], hyi = (T)st->geom.hi[1], hzi = (T)st->geom.hi[2];
+    for (int t = e; t < 3 * nz; t += gridDim.x * 256) wake_line[t] = 0ull;
+  if (e >= nx * ny * nz) return;
+  const T* phi = (const T*)mm.phi;
+  const T hxi = (T)mm.st->geom.hi[0], hyi = (T)mm.st->geom.hi[1], hzi = (T)mm.st->geom.hi[2];
   const T half = (T)0.5;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < G;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % nx);
-    const int j = (int)((e / nx) % ny);
-    const int k = (int)(e / ((long long)nx * ny));
-    const long long sy = nx, sz = (long long)nx * ny;
-    T ex, ey, ez;
-    if (i == 0) ex = hxi * (phi[e] - phi[e + 1]);
-    else if (i == nx - 1) ex = hxi * (phi[e - 1] - phi[e]);
-    else ex = half * hxi * (phi[e - 1] - phi[e + 1]);
-    if (j == 0) ey = hyi * (phi[e] - phi[e + sy]);
-    else if (j == ny - 1) ey = hyi * (phi[e - sy] - phi[e]);
-    else ey = half * hyi * (phi[e - sy] - phi[e + sy]);
-    if (k == 0) ez = hzi * (phi[e] - phi[e + sz]);
-    else if (k == nz - 1) ez = hzi * (phi[e - sz] - phi[e]);
-    else ez = half * hzi * (phi[e - sz] - phi[e + sz]);
-    if (wake) {
-      ex = ex + (T)wake[k];
-      ey = ey + (T)wake[nz + k];
-      ez = ez + (T)wake[2 * nz + k];
-    }
-    rho[e] = 0ull;  // the next deposit accumulates into a cleared charge grid
-    T* o = E + 4 * e;
-    o[0] = ex;
-    o[1] = ey;
-    o[2] = ez;
-    o[3] = (T)0;
+  const int i = e & (nx - 1), j = (e >> (d.lx - 1)) & (ny - 1), k = e >> (d.lx + d.ly - 2);
+  const int sy = nx, sz = nx * ny;
+  const T c = phi[e];
+  const T xm = i > 0 ? phi[e - 1] : c, xp = i < nx - 1 ? phi[e + 1] : c;
+  const T ym = j > 0 ? phi[e - sy] : c, yp = j < ny - 1 ? phi[e + sy] : c;
+  const T zm = k > 0 ? phi[e - sz] : c, zp = k < nz - 1 ? phi[e + sz] : c;
+  T ex = (i == 0 || i == nx - 1 ? hxi : half * hxi) * (xm - xp);
+  T ey = (j == 0 || j == ny - 1 ? hyi : half * hyi) * (ym - yp);
+  T ez = (k == 0 || k == nz - 1 ? hzi : half * hzi) * (zm - zp);
+  if (wake) {
+    ex = ex + (T)wake[k];
+    ey = ey + (T)wake[nz + k];
+    ez = ez + (T)wake[2 * nz + k];
   }
-}
-
-template <typename T>
-__global__ void k_efield(int nx, int ny, int nz, const T* __restrict__ phi,
-                         const DevState* st, T* __restrict__ E,
-                         unsigned long long* __restrict__ rho,
-                         const double* __restrict__ wake,
-                         unsigned long long* __restrict__ wake_line) {
-  efield_body<T>(nx, ny, nz, phi, st, E, rho, wake, wake_line);
-}
-
-template <typename T>
-__global__ void k_efield_group(int nx, int ny, int nz, const PoissonMember* __restrict__ mem) {
-  const PoissonMember& m = mem[blockIdx.y];
-  efield_body<T>(nx, ny, nz, (const T*)m.phi, m.st, (T*)m.efield, m.rho, nullptr, nullptr);
+  mm.rho[e] = 0ull;  // the next deposit accumulates into a cleared charge grid
+  store_field((T*)mm.efield, e, ex, ey, ez);
 }
 
 }  // namespace impz
