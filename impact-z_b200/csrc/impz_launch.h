@@ -124,9 +124,27 @@ cudaError_t launch_conv_group_forward(int nx, int ny, int nz, const PoissonMembe
 template <typename T>
 cudaError_t launch_conv_group_rest(int nx, int ny, int nz, const PoissonMember* mem, int nmem,
                                    cudaStream_t s);
-// true when every Poisson kernel of the form fits the device's shared memory
 template <typename T>
-bool poisson_fits(int nx, int ny, int nz);
+cudaError_t launch_efield_group(int nx, int ny, int nz, const PoissonMember* mem, int nmem,
+                                cudaStream_t s);
+
+#define IMPZ_DECLARE_POISSON(T)                                                                   \
+  template <> int fft_twiddles<T>(int, void*);                                                    \
+  template <> cudaError_t launch_green<T>(const PoissonBuffers&, cudaStream_t);                   \
+  template <> cudaError_t launch_convolve<T>(const PoissonBuffers&, cudaStream_t);                \
+  template <> cudaError_t launch_conv_forward<T>(const PoissonBuffers&, cudaStream_t);            \
+  template <> cudaError_t launch_conv_rest<T>(const PoissonBuffers&, cudaStream_t);               \
+  template <> cudaError_t launch_efield<T>(const PoissonBuffers&, cudaStream_t);                  \
+  template <> cudaError_t launch_green_group<T>(int, int, int, const PoissonMember*, int,         \
+                                                cudaStream_t);                                    \
+  template <> cudaError_t launch_conv_group_forward<T>(int, int, int, const PoissonMember*, int,  \
+                                                       cudaStream_t);                             \
+  template <> cudaError_t launch_conv_group_rest<T>(int, int, int, const PoissonMember*, int,     \
+                                                    cudaStream_t);                                \
+  template <> cudaError_t launch_efield_group<T>(int, int, int, const PoissonMember*, int,        \
+                                                 cudaStream_t);
+IMPZ_DECLARE_POISSON(float)
+IMPZ_DECLARE_POISSON(double)
 
 // Records a CUDA failure for impz_last_cuda_error and returns IMPZ_ERR_CUDA
 // (for translation units other than the C-ABI core).
