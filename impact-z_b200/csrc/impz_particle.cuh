@@ -1753,9 +1753,20 @@ __global__ void __launch_bounds__(BLOCK) k_scan_packed(const ScanArgs* __restric
 // the transverse wake x*ab, x*(1-ab) and the same in y.  The sums are int64
 // fixed point: the density in units of 2^-fixbits, the moments in units of
 // 2^-fixbits of the smallest power of two above the grid's largest |x|
-// (|y|), so they do not depend on the order of the additions.  Sorted
-// particles put a warp mostly on one plane: such a warp adds each sum with
-// one global atomic, any other warp lane by lane.
+// (|y|), so they do not depend on the order of the additions.  Each warp
+// takes a run of IMPZ_WAKE_RUN consecutive particles per lane: sorted
+// particles stay on one plane (or a brick's four) for long, so the lanes add
+// up in registers while the whole warp is on one plane and add the warp's sum
+// with one global atomic per quantity when it leaves it.  A warp on several
+// planes adds up each of the first IMPZ_WAKE_SPLIT of them in turn, the
+// lanes of any other plane one by one.  Reducing and adding every 32
+// particles, lane by lane where they lay on several planes, put all warps on
+// a few addresses: with the field kernel below 87 us of every step at 5e5
+// particles, 128 planes and the transverse sums, now 38 (both in the event
+// profile).
+#define IMPZ_WAKE_RUN 4
+#define IMPZ_WAKE_SPLIT 6
+#define IMPZ_WAKE_PLANES 8  // planes (warps) per block of k_wake_field
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_wake_line(WakeArgs a) {
   const DevState* st = a.st;
@@ -1777,48 +1788,92 @@ __global__ void __launch_bounds__(BLOCK) k_wake_line(WakeArgs a) {
   const double sx = ldexp(1.0, a.fixbits - ex), sy = ldexp(1.0, a.fixbits - ey);
   const int nq = tr ? 6 : 2;
   const int lane = threadIdx.x & 31;
-  for (long long base = (long long)blockIdx.x * BLOCK + (threadIdx.x & ~31); base < n;
-       base += (long long)gridDim.x * BLOCK) {
-    const long long i = base + lane;
-    int kz = -1;
-    long long q[6] = {0, 0, 0, 0, 0, 0};
-    if (i < n) {
-      Particle p;
-      p.x = a.in[0][i]; p.px = a.in[1][i]; p.y = a.in[2][i];
-      p.py = a.in[3][i]; p.ph = a.in[4][i]; p.pt = a.in[5][i];
-      const TFrame t = a.tframe ? stored_tframe(p, gam) : to_tframe(p, gam, rad, a.xl);
-      if (!t.lost) {
-        const int iizz = (int)((t.zt - zmin) / hzw + 1);
-        const double ab = ((zmin - t.zt) + iizz * hzw) / hzw;
-        if (iizz >= 1 && iizz < nz) {
-          kz = iizz - 1;
-          q[0] = llrint(ab * sc);
-          q[1] = llrint((1.0 - ab) * sc);
-          if (tr) {
-            q[2] = llrint(t.xt * ab * sx);
-            q[3] = llrint(t.xt * (1.0 - ab) * sx);
-            q[4] = llrint(t.yt * ab * sy);
-            q[5] = llrint(t.yt * (1.0 - ab) * sy);
+  const long long seg = 32 * IMPZ_WAKE_RUN;
+  long long acc[6] = {0, 0, 0, 0, 0, 0};
+  int plane = -1;  // of the sums in acc (the warp's)
+  auto flush = [&]() {
+    if (plane < 0) return;
+#pragma unroll
+    for (int c = 0; c < 6; c++) {
+      if (c >= nq) break;
+      const long long v = warp_sum_ll(acc[c]);
+      if (lane == 0)
+        atomicAdd(a.line + (long long)(c >> 1) * nz + plane + (c & 1), (unsigned long long)v);
+      acc[c] = 0;
+    }
+    plane = -1;
+  };
+  const long long warps = (long long)gridDim.x * (BLOCK / 32);
+  for (long long w = (long long)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5); w * seg < n;
+       w += warps) {
+    for (long long base = w * seg; base < n && base < (w + 1) * seg; base += 32) {
+      const long long i = base + lane;
+      int kz = -1;
+      long long q[6] = {0, 0, 0, 0, 0, 0};
+      if (i < n) {
+        double xt, yt, zt;
+        bool lost;
+        if (a.tframe) {  // stored in conv1st's frame: three columns suffice
+          xt = a.in[0][i];
+          yt = a.in[2][i];
+          zt = a.in[4][i];
+          lost = isnan(zt);
+        } else {
+          Particle p;
+          p.x = a.in[0][i]; p.px = a.in[1][i]; p.y = a.in[2][i];
+          p.py = a.in[3][i]; p.ph = a.in[4][i]; p.pt = a.in[5][i];
+          const TFrame t = to_tframe(p, gam, rad, a.xl);
+          xt = t.xt; yt = t.yt; zt = t.zt;
+          lost = t.lost;
+        }
+        if (!lost) {
+          const int iizz = (int)((zt - zmin) / hzw + 1);
+          const double ab = ((zmin - zt) + iizz * hzw) / hzw;
+          if (iizz >= 1 && iizz < nz) {
+            kz = iizz - 1;
+            q[0] = llrint(ab * sc);
+            q[1] = llrint((1.0 - ab) * sc);
+            if (tr) {
+              q[2] = llrint(xt * ab * sx);
+              q[3] = llrint(xt * (1.0 - ab) * sx);
+              q[4] = llrint(yt * ab * sy);
+              q[5] = llrint(yt * (1.0 - ab) * sy);
+            }
           }
         }
       }
-    }
-    const int kmin = __reduce_min_sync(0xffffffffu, kz < 0 ? INT_MAX : kz);
-    const int kmax = __reduce_max_sync(0xffffffffu, kz);
-    if (kmax < 0) continue;
-    if (kmin == kmax) {
-      for (int c = 0; c < nq; c++) {
-        long long v = q[c];
+      const int kmin = __reduce_min_sync(0xffffffffu, kz < 0 ? INT_MAX : kz);
+      const int kmax = __reduce_max_sync(0xffffffffu, kz);
+      if (kmax < 0) continue;
+      if (kmin == kmax) {
+        if (plane != kmin) {
+          flush();
+          plane = kmin;
+        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0)
-          atomicAdd(a.line + (long long)(c >> 1) * nz + kmin + (c & 1), (unsigned long long)v);
+        for (int c = 0; c < 6; c++) acc[c] += q[c];
+      } else {
+        // plane by plane (a brick has four), then the lanes that are left
+        unsigned todo = __ballot_sync(0xffffffffu, kz >= 0);
+        for (int r = 0; r < IMPZ_WAKE_SPLIT && todo; r++) {
+          const int k = __shfl_sync(0xffffffffu, kz, __ffs(todo) - 1);
+          const bool mine = kz == k;
+#pragma unroll
+          for (int c = 0; c < 6; c++) {
+            if (c >= nq) break;
+            const long long v = warp_sum_ll(mine ? q[c] : 0);
+            if (lane == 0)
+              atomicAdd(a.line + (long long)(c >> 1) * nz + k + (c & 1), (unsigned long long)v);
+          }
+          todo &= ~__ballot_sync(0xffffffffu, mine);
+        }
+        if (todo >> lane & 1u)
+          for (int c = 0; c < nq; c++)
+            atomicAdd(a.line + (long long)(c >> 1) * nz + kz + (c & 1), (unsigned long long)q[c]);
       }
-    } else if (kz >= 0) {
-      for (int c = 0; c < nq; c++)
-        atomicAdd(a.line + (long long)(c >> 1) * nz + kz + (c & 1), (unsigned long long)q[c]);
     }
   }
+  flush();
 }
 
 // greenwake of wakefieldread_FieldQuant (Field.f90:818-830): the table at
@@ -2076,23 +2131,27 @@ struct AnalyticWake {
 //   conv_z(k) = 0.5 W(0) d(k) + sum_{m>k} d(m) W((m-k) hz),
 // evaluated here directly, and the transverse ones (zero at 0 too)
 // conv_x(k) = sum_{m>k} d(m) xbar(m) Wx((m-k) hz).  Every block builds the
-// density in shared memory; each thread then owns one plane.  The line sums
-// are cleared by the field kernel that follows.
-__global__ void __launch_bounds__(256) k_wake_field(WakeArgs a) {
+// density in shared memory; each warp then owns one plane, its lanes the
+// terms m = k + 1 + lane, + 32, ... (a thread per plane walked up to Nz terms
+// in a chain, in one block for Nz <= 256: 18 us at 128 planes).  The line
+// sums are cleared by the field kernel that follows.
+__global__ void __launch_bounds__(IMPZ_WAKE_PLANES * 32) k_wake_field(WakeArgs a) {
   extern __shared__ double wsm[];
   const int nz = a.nz;
   const DevState* st = a.st;
   const int s = a.fixed_step >= 0 ? a.fixed_step : st->step;
   const StepParams& sp = a.steps[s];
-  const int kk = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int k = blockIdx.x * IMPZ_WAKE_PLANES + (threadIdx.x >> 5);  // the warp's plane
   if (!sp.csr && !sp.wake) {
-    if (kk < nz) a.wfield[kk] = a.wfield[nz + kk] = a.wfield[2 * nz + kk] = 0.0;
+    if (k < nz && lane == 0) a.wfield[k] = a.wfield[nz + k] = a.wfield[2 * nz + k] = 0.0;
     return;
   }
   const bool csr = sp.csr != 0;
   const bool analytic = !csr && sp.wake == 2;
   const bool tr = analytic || (!csr && sp.wake == 1 && a.transverse);
-  const AnalyticWake aw = AnalyticWake::of(sp.wk_aa, sp.wk_gg, sp.wk_len, a.k.Clight);
+  AnalyticWake aw = {};
+  if (analytic) aw = AnalyticWake::of(sp.wk_aa, sp.wk_gg, sp.wk_len, a.k.Clight);
   double* d = wsm;
   double* dx = wsm + nz;
   double* dy = wsm + 2 * nz;
@@ -2134,11 +2193,11 @@ __global__ void __launch_bounds__(256) k_wake_field(WakeArgs a) {
     }
   }
   __syncthreads();
-  const int k = kk;
   if (k >= nz) return;
   double xycon, tcon;
   kick_consts(a.k, gam, cur, xycon, tcon);
   if (csr) {
+    if (lane != 0) return;
     const double zwkmin = st->geom.range[4] / gam + sp.csr_s0;
     const double ez = csr_node(k + 1, d, sp.csr_r0, zwkmin, hzw, sp.csr_blen, gam);
     a.wfield[k] = 0.0;
@@ -2157,16 +2216,20 @@ __global__ void __launch_bounds__(256) k_wake_field(WakeArgs a) {
   // greenwake(1) = 0.5 W(0), in each form as the reference writes it
   const double g0 = analytic ? aw.w0_half(a.k.Clight) : 0.5 * gz[0];
   const double scale = analytic ? 1.0 : a.scale;
-  double cz = d[k] * g0, cx = 0.0, cy = 0.0;
-  if (tr) {
-    for (int m = k + 1; m < nz; m++) {
-      cz = cz + d[m] * gz[m - k];
+  double cz = lane == 0 ? d[k] * g0 : 0.0, cx = 0.0, cy = 0.0;
+  for (int m = k + 1 + lane; m < nz; m += 32) {
+    cz = cz + d[m] * gz[m - k];
+    if (tr) {
       cx = cx + dx[m] * gx[m - k];
       cy = cy + dy[m] * gy[m - k];
     }
-  } else {
-    for (int m = k + 1; m < nz; m++) cz = cz + d[m] * gz[m - k];
   }
+  cz = warp_sum(cz);
+  if (tr) {
+    cx = warp_sum(cx);
+    cy = warp_sum(cy);
+  }
+  if (lane != 0) return;
   const double ezwake = scale * (-cz * hzw);
   const double exwake = scale * (cx * hzw);
   const double eywake = scale * (cy * hzw);

@@ -122,7 +122,8 @@ cudaError_t launch_wake(const WakeArgs& a, int grid, cudaStream_t s) {
   k_wake_line<IMPZ_WAKE_BLOCK><<<grid, IMPZ_WAKE_BLOCK, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_wake_field<<<(a.nz + 255) / 256, 256, (size_t)6 * a.nz * sizeof(double), s>>>(a);
+  k_wake_field<<<(a.nz + IMPZ_WAKE_PLANES - 1) / IMPZ_WAKE_PLANES, IMPZ_WAKE_PLANES * 32,
+                 (size_t)6 * a.nz * sizeof(double), s>>>(a);
   return cudaGetLastError();
 }
 
