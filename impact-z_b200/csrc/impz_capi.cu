@@ -411,7 +411,7 @@ struct impz_bunch_s {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t stream2 = nullptr;   // Green-function build, overlapped with the deposit
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_dep = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_dep = nullptr, ev_scan = nullptr;
   bool serial_green = false;
   int form = 0, flags = 0;
   long long cap = 0;
@@ -715,8 +715,11 @@ int field_step(impz_bunch_t b, const StepParams* table, int fixed) {
     CK(launch_deposit(b, d));
   }
   // the scan of the counts is needed only by the push: on the second stream
-  // it runs beside the forward transform
+  // it runs beside the transforms, which wait for the Green build alone (a
+  // bunch of 1e5 particles builds its Green function as long as it deposits,
+  // so waiting for the scan too put its 6 us on the step)
   if (!serial) {
+    CK(cudaEventRecord(b->ev_join, b->stream2));
     CK(cudaEventRecord(b->ev_dep, b->stream));
     CK(cudaStreamWaitEvent(b->stream2, b->ev_dep, 0));
   }
@@ -724,7 +727,7 @@ int field_step(impz_bunch_t b, const StepParams* table, int fixed) {
     ProfScope ps(b, IMPZ_PROF_SCAN, 1, gs);
     CK(exact::launch_scan(b->counts, b->cursor, b->bsum, b->G + 1, b->st, gs));
   }
-  if (!serial) CK(cudaEventRecord(b->ev_join, b->stream2));
+  if (!serial) CK(cudaEventRecord(b->ev_scan, b->stream2));
   if (b->run_wake) {
     ProfScope ps(b, IMPZ_PROF_WAKE, 2);
     CK(exact::launch_wake(wake_args(b, table, fixed), b->grid_wake, b->stream));
@@ -741,7 +744,9 @@ int field_step(impz_bunch_t b, const StepParams* table, int fixed) {
     if (b->f32()) { CK(launch_conv_rest<float>(pb, b->stream)); }
     else { CK(launch_conv_rest<double>(pb, b->stream)); }
   }
-  return solve_efield(b);
+  if ((r = solve_efield(b))) return r;
+  if (!serial) CK(cudaStreamWaitEvent(b->stream, b->ev_scan, 0));
+  return IMPZ_OK;
 }
 
 int upload_fine(impz_bunch_t b, const StepParams* host2) {
@@ -963,6 +968,7 @@ void free_bunch(impz_bunch_t b) {
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
   if (b->ev_join) cudaEventDestroy(b->ev_join);
   if (b->ev_dep) cudaEventDestroy(b->ev_dep);
+  if (b->ev_scan) cudaEventDestroy(b->ev_scan);
   if (b->stream2) cudaStreamDestroy(b->stream2);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
@@ -1064,6 +1070,7 @@ int impz_bunch_create(const double* pts, long long n, double current, double mas
   ALLOC(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
   ALLOC(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
   ALLOC(cudaEventCreateWithFlags(&b->ev_dep, cudaEventDisableTiming));
+  ALLOC(cudaEventCreateWithFlags(&b->ev_scan, cudaEventDisableTiming));
   const Layout L = plan_layout(n, nx, ny, nz, form, flags);
   ALLOC(cudaMalloc((void**)&b->arena, L.total));
   char* base = b->arena;
@@ -2033,7 +2040,11 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
               : exact::launch_deposit_packed(d_dep + (size_t)p * nb, d_do, nb, n_dep, species,
                                              s);
       if (e != cudaSuccess) return e;
-      if ((e = exact::launch_scan_packed(d_scn, d_so, nb, n_scan, s)) != cudaSuccess) return e;
+      // the count scan beside the transforms; the push waits for it
+      if ((e = cudaEventRecord(b0->ev_dep, s)) != cudaSuccess) return e;
+      if ((e = cudaStreamWaitEvent(s2, b0->ev_dep, 0)) != cudaSuccess) return e;
+      if ((e = exact::launch_scan_packed(d_scn, d_so, nb, n_scan, s2)) != cudaSuccess) return e;
+      if ((e = cudaEventRecord(b0->ev_scan, s2)) != cudaSuccess) return e;
       for (const BatchGroup& g : groups) {
         e = f32 ? launch_conv_group_forward<float>(g.nx, g.ny, g.nz, d_mem + g.first, g.count, s)
                 : launch_conv_group_forward<double>(g.nx, g.ny, g.nz, d_mem + g.first, g.count,
@@ -2050,6 +2061,7 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
         if (e != cudaSuccess) return e;
       }
       g_launches += nlaunch_sc - 1;
+      if ((e = cudaStreamWaitEvent(s, b0->ev_scan, 0)) != cudaSuccess) return e;
     }
     const AdvanceArgs* a = d_adv + (size_t)(sc ? p : 2 + p) * nb;
     e = f32 ? fast::launch_advance_packed(a, d_ao, nb, n_adv, true, light, species, s)
@@ -2118,8 +2130,10 @@ static size_t packed_scratch_bytes(int nb) {
          3 * round_up((size_t)(nb + 1) * sizeof(int), kAlign);
 }
 
-static int packed_step(impz_bunch_t* bs, int nb, cudaStream_t s, cudaStream_t s2,
-                       cudaEvent_t evf, cudaEvent_t evj, char* dscratch, bool f32, bool light) {
+static int packed_step(impz_bunch_t* bs, int nb, char* dscratch, bool f32, bool light) {
+  const impz_bunch_t b0 = bs[0];  // its streams and events carry the packed launches
+  cudaStream_t s = b0->stream, s2 = b0->stream2;
+  cudaEvent_t evf = b0->ev_fork, evj = b0->ev_join;
   std::vector<impz_bunch_t> mem_b, sc_b;
   bool species = false;  // a member carries the species column
   for (int i = 0; i < nb; i++) {
@@ -2200,9 +2214,13 @@ static int packed_step(impz_bunch_t* bs, int nb, cudaStream_t s, cudaStream_t s2
     e = f32 ? fast::launch_deposit_packed(d_dep, d_do, ns, dep_offs[ns], species, s)
             : exact::launch_deposit_packed(d_dep, d_do, ns, dep_offs[ns], species, s);
     if (e != cudaSuccess) return cuda_fail(e, "packed step: deposit");
+    // the count scan beside the transforms; the push waits for it
+    CK(cudaEventRecord(b0->ev_dep, s));
+    CK(cudaStreamWaitEvent(s2, b0->ev_dep, 0));
     e = exact::launch_scan_packed((const ScanArgs*)(dscratch + o_scn),
-                                  (const int*)(dscratch + o_so), ns, scan_offs[ns], s);
+                                  (const int*)(dscratch + o_so), ns, scan_offs[ns], s2);
     if (e != cudaSuccess) return cuda_fail(e, "packed step: scan");
+    CK(cudaEventRecord(b0->ev_scan, s2));
     for (const BatchGroup& g : groups) {
       e = f32 ? launch_conv_group_forward<float>(g.nx, g.ny, g.nz, d_mem + g.first, g.count, s)
               : launch_conv_group_forward<double>(g.nx, g.ny, g.nz, d_mem + g.first, g.count, s);
@@ -2218,6 +2236,7 @@ static int packed_step(impz_bunch_t* bs, int nb, cudaStream_t s, cudaStream_t s2
       if (e != cudaSuccess) return cuda_fail(e, "packed step: field solve");
     }
     g_launches += 2 + 9 * (int)groups.size();
+    CK(cudaStreamWaitEvent(s, b0->ev_scan, 0));
   }
   e = f32 ? fast::launch_advance_packed((const AdvanceArgs*)(dscratch + o_adv),
                                         (const int*)(dscratch + o_ao), nm, adv_offs[nm], true,
@@ -2274,8 +2293,7 @@ int impz_run_advance_packed(impz_bunch_t* bunches, int nb, int steps, int* remai
   CK(cudaMallocAsync((void**)&dscratch, packed_scratch_bytes(np), s));
   int r = IMPZ_OK;
   for (int k = 0; k < steps && !r; k++)
-    r = packed_step(pk.data(), np, s, pk[0]->stream2, pk[0]->ev_fork, pk[0]->ev_join, dscratch,
-                    b0->f32(), light);
+    r = packed_step(pk.data(), np, dscratch, b0->f32(), light);
   cudaFreeAsync(dscratch, s);
   CK(cudaEventRecord(pk[0]->ev_dep, s));
   for (int i = 1; i < np; i++) CK(cudaStreamWaitEvent(pk[i]->stream, pk[0]->ev_dep, 0));
