@@ -463,15 +463,15 @@ struct impz_bunch_s {
   double sc_gam = 0, sc_rad = 0;
   // last impz_run_async
   CompiledLattice lat;
-  bool run_light = false;  // the run's programs need only the light particle pass
+  bool run_light = false;  // every step of the run needs only the light particle pass
   bool run_pending = false;
   size_t bytes = 0;
-  // graphs of two space-charge steps, per start parity
-  cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  const StepParams* g_steps[2] = {nullptr, nullptr};
-  const double* g_mom[2] = {nullptr, nullptr};
-  bool g_light[2] = {false, false};  // which particle pass the graph holds
-  int g_wake[2] = {-1, -1};          // wake generation the graph holds
+  // graphs of two space-charge steps, per start parity and particle pass
+  // (graph 2 parity + light), and the buffers and wake generation each holds
+  cudaGraphExec_t gexec[4] = {nullptr, nullptr, nullptr, nullptr};
+  const StepParams* g_steps[4] = {nullptr, nullptr, nullptr, nullptr};
+  const double* g_mom[4] = {nullptr, nullptr, nullptr, nullptr};
+  int g_wake[4] = {-1, -1, -1, -1};
   // read-in wakefield (impz_wake_set): table [3][ntab], then the line sums
   // [3][nz] and the per-plane field [3][nz] in one allocation
   bool wk_on = false, wk_tr = false;
@@ -490,7 +490,7 @@ struct impz_bunch_s {
   // the last per-step kick, grown as needed
   double* lzd = nullptr;
   size_t lzd_cap = 0;
-  const double* g_lzd[2] = {nullptr, nullptr};  // the data the step graphs point to
+  const double* g_lzd[4] = {nullptr, nullptr, nullptr, nullptr};  // the data the step graphs point to
   int run_next = 0;       // next step of the run in progress
   double run_z = 0;       // z and refptcl at the end of the run in progress
   double run_ref[6] = {0};
@@ -611,11 +611,17 @@ bool program_is_light(const MapProgram& prog) {
   return true;
 }
 
+// whether the light particle pass can run step sp: drifts and block-diagonal
+// maps, no Lorentz kick (in the full pass only).  Chosen step by step: the
+// full pass spills registers and takes 1.8 times as long, and a lattice's
+// bends, cavities or K-map quadrupoles are often a few steps among many drifts
+bool step_is_light(const StepParams& sp) {
+  return !sp.lorentz && program_is_light(sp.post) && program_is_light(sp.pre_next);
+}
+
 bool table_is_light(const std::vector<StepParams>& steps) {
   for (const StepParams& sp : steps)
-    if (sp.lorentz) return false;  // the Lorentz kick is in the full pass only
-  for (const StepParams& sp : steps)
-    if (!program_is_light(sp.post) || !program_is_light(sp.pre_next)) return false;
+    if (!step_is_light(sp)) return false;
   return true;
 }
 
@@ -901,7 +907,7 @@ int build_species(impz_bunch_t b, const double* pts, long long n) {
   // the step graphs hold the weight (field scale), q/m and the number of
   // species by value
   if (b->weight != wref || b->sp.qmi != qm[0] || b->nspecies != (int)qm.size())
-    for (int p = 0; p < 2; p++)
+    for (int p = 0; p < 4; p++)
       if (b->gexec[p]) {
         cudaGraphExecDestroy(b->gexec[p]);
         b->gexec[p] = nullptr;
@@ -962,7 +968,7 @@ void free_bunch(impz_bunch_t b) {
   if (b->wk_mem) cudaFree(b->wk_mem);
   if (b->lzd) cudaFree(b->lzd);
   for (cudaEvent_t e : b->ev_pool) cudaEventDestroy(e);
-  for (int p = 0; p < 2; p++)
+  for (int p = 0; p < 4; p++)
     if (b->gexec[p]) cudaGraphExecDestroy(b->gexec[p]);
   if (b->stream2) cudaStreamSynchronize(b->stream2);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -1334,7 +1340,7 @@ static int run_fine_advance(impz_bunch_t b, const StepParams host[2], int kick, 
   int r = upload_fine(b, host);
   if (r) return r;
   AdvanceArgs a = advance_args(b, b->dfine, 0, kick, post, pre, b->mom_fine, 0);
-  CK(launch_adv(b, a, false));
+  CK(launch_adv(b, a, step_is_light(host[0])));
   if (kick) b->parity ^= 1;
   if (rec) {
     CK(cudaMemcpyAsync(rec, b->mom_fine, IMPZ_MOMREC * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1712,13 +1718,13 @@ int impz_bunch_upload(impz_bunch_t b, const double* pts, long long n, double cur
 
 // ---- whole-lattice runner --------------------------------------------
 // One step s (read from DevState::step on the device) as direct launches.
-static int launch_step(impz_bunch_t b, bool sc) {
+static int launch_step(impz_bunch_t b, bool sc, bool light) {
   if (sc) {
     int r = field_step(b, b->dsteps, -1);
     if (r) return r;
   }
   AdvanceArgs a = advance_args(b, b->dsteps, -1, sc ? 1 : 0, 1, 1, b->mom_out, 0);
-  CK(launch_adv(b, a, b->run_light));
+  CK(launch_adv(b, a, light));
   if (sc) b->parity ^= 1;
   return IMPZ_OK;
 }
@@ -1767,22 +1773,21 @@ static int wake_alloc(impz_bunch_t b, int ntab) {
 static int wake_key(impz_bunch_t b) { return 2 * b->wk_gen + (b->run_wake ? 1 : 0); }
 
 // Two space-charge steps captured as one CUDA graph (parity returns to its
-// start value), cached per start parity and re-captured when the step table
-// or the record buffer move.
-static int graph_pair(impz_bunch_t b) {
-  const int p = b->parity;
-  if (b->gexec[p] && (b->g_steps[p] != b->dsteps || b->g_mom[p] != b->mom_out ||
-                      b->g_light[p] != b->run_light || b->g_wake[p] != wake_key(b) ||
-                      b->g_lzd[p] != b->lzd)) {
-    cudaGraphExecDestroy(b->gexec[p]);
-    b->gexec[p] = nullptr;
+// start value), cached per start parity and particle pass and re-captured
+// when the step table or the record buffer move.
+static int graph_pair(impz_bunch_t b, bool light) {
+  const int p = b->parity, k = 2 * p + (light ? 1 : 0);
+  if (b->gexec[k] && (b->g_steps[k] != b->dsteps || b->g_mom[k] != b->mom_out ||
+                      b->g_wake[k] != wake_key(b) || b->g_lzd[k] != b->lzd)) {
+    cudaGraphExecDestroy(b->gexec[k]);
+    b->gexec[k] = nullptr;
   }
-  if (!b->gexec[p]) {
+  if (!b->gexec[k]) {
     cudaGraph_t g = nullptr;
     const long long counted = g_launches.load();
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    int r = launch_step(b, true);
-    if (!r) r = launch_step(b, true);
+    int r = launch_step(b, true, light);
+    if (!r) r = launch_step(b, true, light);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     g_launches = counted;  // capture recorded the launches without running them
     if (r) {
@@ -1790,18 +1795,17 @@ static int graph_pair(impz_bunch_t b) {
       return r;
     }
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-    e = cudaGraphInstantiate(&b->gexec[p], g, 0);
+    e = cudaGraphInstantiate(&b->gexec[k], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-    b->g_steps[p] = b->dsteps;
-    b->g_mom[p] = b->mom_out;
-    b->g_light[p] = b->run_light;
-    b->g_wake[p] = wake_key(b);
-    b->g_lzd[p] = b->lzd;
+    b->g_steps[k] = b->dsteps;
+    b->g_mom[k] = b->mom_out;
+    b->g_wake[k] = wake_key(b);
+    b->g_lzd[k] = b->lzd;
     b->parity = p;  // capture did not execute anything
   }
   g_launches += 2 * (12 + (b->run_wake ? 2 : 0));
-  CK(cudaGraphLaunch(b->gexec[p], b->stream));
+  CK(cudaGraphLaunch(b->gexec[k], b->stream));
   return IMPZ_OK;
 }
 
@@ -1836,7 +1840,7 @@ static int run_begin(impz_bunch_t b, const impz_elem_t* elems, int nelem) {
   CK(cudaMemcpyAsync(&b->st->step, &b->h_step0, sizeof(int), cudaMemcpyHostToDevice,
                      b->stream));
   AdvanceArgs a = advance_args(b, b->dsteps, -1, 0, 1, 1, b->mom_out, 0);
-  CK(launch_adv(b, a, b->run_light));
+  CK(launch_adv(b, a, step_is_light(L.steps[0])));
   b->run_next = 1;
   return IMPZ_OK;
 }
@@ -1850,14 +1854,15 @@ static int run_advance(impz_bunch_t b, int budget) {
   int done = 0;
   while (b->run_next <= K && (done == 0 || done < budget)) {
     const int s = b->run_next;
-    const bool sc = L.steps[s].sc != 0;
+    const bool sc = L.steps[s].sc != 0, light = step_is_light(L.steps[s]);
     int r;
-    if (!b->prof_on && sc && s + 1 <= K && L.steps[s + 1].sc) {
-      r = graph_pair(b);
+    if (!b->prof_on && sc && s + 1 <= K && L.steps[s + 1].sc &&
+        step_is_light(L.steps[s + 1]) == light) {
+      r = graph_pair(b, light);
       b->run_next += 2;
       done += 2;
     } else {
-      r = launch_step(b, sc);
+      r = launch_step(b, sc, light);
       b->run_next += 1;
       done += 1;
     }
@@ -2461,7 +2466,7 @@ int impz_set_integrator(impz_bunch_t b, int flagmap) {
 
 static void drop_graphs(impz_bunch_t b) {
   cudaStreamSynchronize(b->stream);
-  for (int p = 0; p < 2; p++)
+  for (int p = 0; p < 4; p++)
     if (b->gexec[p]) {
       cudaGraphExecDestroy(b->gexec[p]);
       b->gexec[p] = nullptr;
