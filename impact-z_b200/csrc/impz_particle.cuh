@@ -1341,6 +1341,55 @@ __global__ void __launch_bounds__(BLOCK, IMPZ_ADV_MINB)
 }
 
 // ---------------------------------------------------------------------
+// A particle's fixed-point deposit on its cell's eight corners, in the order
+// of deposit_BeamBunch (BeamBunch.f90:3749-3763): corner k gets
+// round(w_k 2^f), and the corner of the largest weight what is missing to one
+// unit, 2^f (punit).  The rounding adds 1.5 2^52, which leaves the integer in
+// the low bits of the double: sh[k] is that bit pattern, quanta + kMagicBits.
+// The missing rest (a few quanta of either sign) follows from the low words
+// alone; the largest weight is the product of each axis's larger half, `big`
+// its corner (ties to the lower node, as the first of equal weights).
+// pscale = 2^f, or 2^f times the particle's relative weight.
+constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
+constexpr long long kMagicBits = 0x4338000000000000ll;
+
+struct Corners {
+  unsigned long long sh[8];
+  int rest;              // 2^f minus the rounded corners' sum
+  bool hi_x, hi_y, hi_z;  // the largest weight's node is the upper one
+};
+
+__device__ __forceinline__ Corners corner_quanta(double ab, double cd, double ef, double pscale,
+                                                 unsigned punit_lo) {
+  const double ab1 = 1.0 - ab, cd1 = 1.0 - cd, ef1 = 1.0 - ef;
+  const double w8[8] = {ab * cd * ef,   ab * cd1 * ef,   ab * cd1 * ef1,  ab * cd * ef1,
+                        ab1 * cd * ef1, ab1 * cd1 * ef1, ab1 * cd1 * ef,  ab1 * cd * ef};
+  Corners c;
+  unsigned sum = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    c.sh[k] = (unsigned long long)__double_as_longlong(__dadd_rn(__dmul_rn(w8[k], pscale), kMagic));
+    sum += (unsigned)c.sh[k];  // kMagicBits has a zero low word
+  }
+  c.rest = (int)(punit_lo - sum);
+  c.hi_x = ab < ab1;
+  c.hi_y = cd < cd1;
+  c.hi_z = ef < ef1;
+  return c;
+}
+
+// the quanta as 64-bit integers, the rest added to its corner
+__device__ __forceinline__ void corner_sums(const Corners& c, unsigned long long (&q)[8]) {
+  // corner k is the upper node in x for k >= 4, in y for 1, 2, 5, 6, in z for 2, 3, 4, 5
+  const int big = c.hi_x ? (c.hi_y ? (c.hi_z ? 5 : 6) : (c.hi_z ? 4 : 7))
+                         : (c.hi_y ? (c.hi_z ? 2 : 1) : (c.hi_z ? 3 : 0));
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    q[k] = c.sh[k] - (unsigned long long)kMagicBits +
+           (k == big ? (unsigned long long)(long long)c.rest : 0ull);
+}
+
+// ---------------------------------------------------------------------
 // Charge deposit.  Each block takes chunks of BLOCK*U consecutive particles.
 // Particles are kept sorted by the previous step's deposit cell, so after the
 // grid is refitted a chunk still covers a small box of cells, give or take
@@ -1355,19 +1404,20 @@ __global__ void __launch_bounds__(BLOCK, IMPZ_ADV_MINB)
 // copies.  Small boxes (the dense core) thus get many copies, large boxes
 // (sparse regions, few lanes per cell) few.  Each tile word keeps a node's
 // fixed-point sum as two 32-bit halves (the low 20 bits and the rest) so
-// that native 32-bit shared atomics suffice: a chunk of at most 2048
-// particles cannot overflow either half.  With quanta of at most 2^21 (the
-// FP32-convolution form) one word holds a chunk's sum and the high half is
-// not used.  Accumulation is in int64 fixed
+// that native 32-bit shared atomics suffice: a chunk of at most 1024
+// particles cannot overflow either half.  Accumulation is in int64 fixed
 // point (2^-fixbits of a unit macro-particle charge), so the result does not
 // depend on the order of the additions; the corner with the largest weight
 // takes 2^fixbits minus the other seven (never negative), so every live
-// particle deposits exactly one unit.
+// particle deposits exactly one unit.  In the tile the missing rest is one
+// more atomic on the low word of that corner (signed at the flush).  The
+// selects that put it into a corner in registers cost more than it does:
+// 104 us per deposit of 4e6 particles with them, 96 without (509 and 474 us
+// for 2e7 on 64x64x2048).
 #ifndef IMPZ_DEP_RMAX
 #define IMPZ_DEP_RMAX 32
 #endif
 #define IMPZ_DEP_LOBITS 20
-#define IMPZ_DEP_FIXBITS_1WORD 21
 template <int BLOCK, int U, bool SP>
 __device__ __forceinline__ void deposit_pass(const DepositArgs& a, const int vbx, const int vgx) {
   static_assert(BLOCK * U <= 1024, "one-word tile sums sized for chunks of at most 1024");
@@ -1394,15 +1444,9 @@ __device__ __forceinline__ void deposit_pass(const DepositArgs& a, const int vbx
   const long long P = (long long)nx * ny;
   const long long G = P * nz;
   const double scale = ldexp(1.0, a.fixbits);
-  const unsigned long long unit = 1ull << a.fixbits;
-  // round-to-nearest-even of w*2^f (exact below 2^51) by the 1.5*2^52 shift
-  const double magic = 6755399441055744.0;
-  const long long magic_bits = 0x4338000000000000ll;
+  const unsigned unit_lo = (unsigned)(1ull << a.fixbits);
   const unsigned lomask = (1u << IMPZ_DEP_LOBITS) - 1u;
-  // quanta of at most 2^21: a chunk's sum at one node stays below 2^31 in
-  // a single word (species of either sign take the two signed halves)
   const bool species = SP && a.sp_in != nullptr;
-  const bool split = a.fixbits > IMPZ_DEP_FIXBITS_1WORD || species;
   const long long chunk = (long long)BLOCK * U;
   const int lane = threadIdx.x & 31;
   for (long long c0 = (long long)vbx * chunk; c0 < n; c0 += (long long)vgx * chunk) {
@@ -1477,46 +1521,23 @@ __device__ __forceinline__ void deposit_pass(const DepositArgs& a, const int vbx
 #pragma unroll
     for (int u = 0; u < U; u++) {
       if (cell[u] < 0) continue;
-      const double ab = wab[u], cd = wcd[u], ef = wef[u];
-      // weights in the order of deposit_BeamBunch (BeamBunch.f90:3749-3763)
-      const double w8[8] = {ab * cd * ef,
-                            ab * (1.0 - cd) * ef,
-                            ab * (1.0 - cd) * (1.0 - ef),
-                            ab * cd * (1.0 - ef),
-                            (1.0 - ab) * cd * (1.0 - ef),
-                            (1.0 - ab) * (1.0 - cd) * (1.0 - ef),
-                            (1.0 - ab) * (1.0 - cd) * ef,
-                            (1.0 - ab) * cd * ef};
-      int big = 0;
-      double wbig = w8[0];
-#pragma unroll
-      for (int k = 1; k < 8; k++)
-        if (w8[k] > wbig) { wbig = w8[k]; big = k; }
       // a particle of relative weight ws deposits round(ws 2^f) quanta (one
       // unit, 2^f, for the bunch's own species); two's complement for
       // species of the other sign
       double pscale = scale;
-      unsigned long long punit = unit;
+      unsigned punit_lo = unit_lo;
       if (species) {  // the particle's charge weight relative to the bunch's
         const double ws = __ldg(a.sp_w + a.sp_in[c0 + (long long)u * BLOCK + threadIdx.x]);
         pscale = __dmul_rn(ws, scale);
-        punit = (unsigned long long)(__double_as_longlong(__dadd_rn(pscale, magic)) - magic_bits);
+        punit_lo = (unsigned)__double_as_longlong(__dadd_rn(pscale, kMagic));
       }
-      unsigned long long qv[8];
-      unsigned long long sum7 = 0;
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const double sh = __dadd_rn(__dmul_rn(w8[k], pscale), magic);
-        qv[k] = (k == big) ? 0ull : (unsigned long long)(__double_as_longlong(sh) - magic_bits);
-        sum7 += qv[k];
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        if (k == big) qv[k] = punit - sum7;
+      const Corners cq = corner_quanta(wab[u], wcd[u], wef[u], pscale, punit_lo);
       if (!tiled) {
         const long long c = cell[u];
         const long long node[8] = {c, c + nx, c + nx + P, c + P, c + 1 + P, c + 1 + nx + P,
                                    c + 1 + nx, c + 1};
+        unsigned long long qv[8];
+        corner_sums(cq, qv);
 #pragma unroll
         for (int k = 0; k < 8; k++) atomicAdd(a.rho + node[k], qv[k]);
         atomicAdd(a.counts + cell_key((int)(pk[u] & 1023u), (int)((pk[u] >> 10) & 1023u),
@@ -1526,16 +1547,16 @@ __device__ __forceinline__ void deposit_pass(const DepositArgs& a, const int vbx
                       bx * (((int)((pk[u] >> 10) & 1023u) - y0) + by * ((int)(pk[u] >> 20) - z0));
         const int node[8] = {t, t + bx, t + bx + bxy, t + bxy, t + 1 + bxy, t + 1 + bx + bxy,
                              t + 1 + bx, t + 1};
-        if (split) {
+        // the quanta's low 20 bits, and the bits above them: those of the
+        // pattern, less the magic's 0x80000000 there
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
-            atomicAdd(tlo + node[k], (unsigned)(qv[k] & lomask));
-            atomicAdd(thi + node[k], (unsigned)((long long)qv[k] >> IMPZ_DEP_LOBITS));
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 8; k++) atomicAdd(tlo + node[k], (unsigned)qv[k]);
+        for (int k = 0; k < 8; k++) {
+          atomicAdd(tlo + node[k], (unsigned)cq.sh[k] & lomask);
+          atomicAdd(thi + node[k], (unsigned)(cq.sh[k] >> IMPZ_DEP_LOBITS) - 0x80000000u);
         }
+        if (cq.rest)
+          atomicAdd(tlo + t + (cq.hi_x ? 1 : 0) + (cq.hi_y ? bx : 0) + (cq.hi_z ? bxy : 0),
+                    (unsigned)cq.rest);
         atomicAdd(tcnt + t, 1u);
       }
     }
@@ -1546,14 +1567,15 @@ __device__ __forceinline__ void deposit_pass(const DepositArgs& a, const int vbx
         unsigned long long q = 0ull;
         unsigned int k = 0u;
         for (int r = 0, o = e; r < R; r++, o += S) {
-          const unsigned lo = tlo[o], hi = split ? thi[o] : 0u, c = tcnt[o];
+          const unsigned lo = tlo[o], hi = thi[o], c = tcnt[o];
           if (lo | hi | c) {
-            // the high half is signed (a negative quantum's arithmetic shift)
+            // both halves are signed (a negative quantum's arithmetic shift;
+            // a rest below zero)
             q += ((unsigned long long)(long long)(int)hi << IMPZ_DEP_LOBITS) +
-                 (unsigned long long)lo;
+                 (unsigned long long)(long long)(int)lo;
             k += c;
             tlo[o] = 0u;
-            if (split) thi[o] = 0u;
+            thi[o] = 0u;
             tcnt[o] = 0u;
           }
         }

@@ -63,9 +63,8 @@ __global__ void __launch_bounds__(256) k_static_deposit(StaticDepositArgs a,
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const long long P = (long long)nx * ny;
   const double scale = ldexp(1.0, a.fixbits);
-  const unsigned long long unit = 1ull << a.fixbits;
-  const double magic = 6755399441055744.0;  // 1.5 * 2^52: round to nearest even
-  const long long magic_bits = 0x4338000000000000ll;
+  const unsigned unit_lo = (unsigned)(1ull << a.fixbits);
+  griddep_launch();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n;
        i += (long long)gridDim.x * blockDim.x) {
     Particle p;
@@ -75,32 +74,9 @@ __global__ void __launch_bounds__(256) k_static_deposit(StaticDepositArgs a,
     if (t.lost) continue;
     const Cell c = cic_cell(t.xt, t.yt, t.zt, a.g);
     if (!cell_inside(c, nx, ny, nz)) continue;
-    const double ab = c.ab, cd = c.cd, ef = c.ef;
-    // corner order of deposit_BeamBunch (BeamBunch.f90:3749-3763)
-    const double w8[8] = {ab * cd * ef,
-                          ab * (1.0 - cd) * ef,
-                          ab * (1.0 - cd) * (1.0 - ef),
-                          ab * cd * (1.0 - ef),
-                          (1.0 - ab) * cd * (1.0 - ef),
-                          (1.0 - ab) * (1.0 - cd) * (1.0 - ef),
-                          (1.0 - ab) * (1.0 - cd) * ef,
-                          (1.0 - ab) * cd * ef};
-    int big = 0;
-    double wbig = w8[0];
-#pragma unroll
-    for (int k = 1; k < 8; k++)
-      if (w8[k] > wbig) { wbig = w8[k]; big = k; }
     unsigned long long qv[8];
-    unsigned long long sum7 = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const double sh = __dadd_rn(__dmul_rn(w8[k], scale), magic);
-      qv[k] = (k == big) ? 0ull : (unsigned long long)(__double_as_longlong(sh) - magic_bits);
-      sum7 += qv[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (k == big) qv[k] = unit - sum7;
+    corner_sums(corner_quanta(c.ab, c.cd, c.ef, scale, unit_lo), qv);
+    griddep_wait();  // the cells are cleared
     const long long cc = lin_cell(c, nx, ny);
     const long long node[8] = {cc, cc + nx, cc + nx + P, cc + P, cc + 1 + P, cc + 1 + nx + P,
                                cc + 1 + nx, cc + 1};
