@@ -31,8 +31,7 @@
 // of the line index q at ky and the same T at 2Ny - ky), and a group's
 // points lie together, z by z, S[group][z][side][T]: a block reads and
 // writes one contiguous piece, and the xy passes touch whole 32-byte sectors
-// (T = 4 FP32 values).  T is 4, and less where the lines are so long that
-// fewer fit a block (zt_log).  Line q = row * Nx + kx for kx < Nx, and
+// (T = 4 FP32 values, 2 or 4 FP64 ones; zt_log).  Line q = row * Nx + kx for kx < Nx, and
 // Ny * Nx + row for kx = Nx, with row = ky (side 0) or 2Ny - ky (side 1; row
 // 0 holds ky = 0 and ky = Ny).  G-hat holds T lines together in the same
 // way, ((q / T) (Nz+1) + kz) T + q mod T with q = ky Nx + kx, then the kx =
@@ -52,10 +51,13 @@ struct PoissonDims {
   int lx, ly, lz;  // log2 of the doubled lengths 2nx, 2ny, 2nz
 };
 
-// log2 of T, the lines of one side of a group, for z transforms of 2^lz points
+// log2 of T, the lines of one side of a group, for z transforms of 2^lz
+// points.  Never less than a 32-byte sector: with T = 1 for the long lines
+// (as many as the z convolution works on at once) the xy passes moved 8 of
+// every 32 bytes, and took 307 of 501 us at 64x64x2048.
 template <typename T>
 __host__ __device__ constexpr int zt_log(int lz) {
-  return sizeof(T) == 4 ? (lz <= 9 ? 2 : lz == 10 ? 1 : 0) : (lz <= 8 ? 2 : lz == 9 ? 1 : 0);
+  return sizeof(T) == 4 ? 2 : lz <= 8 ? 2 : 1;
 }
 
 // element index of spectrum line (ky, kx) at plane z
@@ -305,14 +307,15 @@ struct ZShape {
 };
 
 // lines of the z convolution in work at once: a whole group, several groups
-// where the lines are short, one line where a block of 1024 threads holds
-// no more (8192 points in FP64)
+// where the lines are short, and a part of the group, round by round, where a
+// block of 512 threads holds no more (the rounds share sectors that stay in
+// L1 or L2)
 template <typename T, int LZ>
 struct ZConv {
   typedef Fft<T, LZ> F;
   static constexpr int lt = zt_log<T>(LZ), NL = 2 << lt;
   static constexpr int GPB = NL * F::TPL >= 128 ? 1 : 128 / (NL * F::TPL);  // groups per block
-  static constexpr int PAR = NL * F::TPL > 1024 ? 1024 / F::TPL : NL * GPB;
+  static constexpr int PAR = NL * F::TPL <= 512 ? NL * GPB : F::TPL >= 512 ? 1 : 512 / F::TPL;
   static constexpr int ROUNDS = NL * GPB / PAR;
   typedef ZShape<T, LZ, PAR> Z;
 };
