@@ -719,6 +719,8 @@ int half_map_ops(const Phys& P, const impz_elem_t& e, double zedge, double z, do
       op.c[0] = refptcl[5]; op.c[1] = gambet0; op.c[2] = beta0;
       op.c[3] = sp.charge / sp.mass; op.c[4] = e.val[0]; op.c[5] = tau;
       op.c[6] = Scxl; op.c[7] = sp.qmi;
+      op.c[8] = gambet0 * e.val[0] / (sp.charge / sp.mass); op.c[9] = 1.0 / Scxl;
+      op.c[10] = 1.0 / beta0; op.c[11] = tau / Scxl;  // c[8..]: the FP32 form's map
       refptcl[4] = refptcl[4] + tau / beta0 / Scxl;
       return push_op(prog, op);
     }
@@ -807,8 +809,10 @@ MapOp pole_op(const Phys& P, MapKind kind, double h0, double h1, double tanphi, 
   const double secphib2 = 1. + tanphib * tanphib;
   const double beta0 = std::sqrt(1.0 - 1.0 / (gam0 * gam0));
   const double gambet = beta0 * gam0;
-  const double c[16] = {h0,      h1,       tanphi,  tanphib, k1,  psi, tanphi2, secphi2,
-                        secphi3, secphib2, beta0,   gambet,  gam0, qm0, sp.qmi, P.Scxl};
+  const double c[20] = {h0,      h1,       tanphi,  tanphib, k1,  psi, tanphi2, secphi2,
+                        secphi3, secphib2, beta0,   gambet,  gam0, qm0, sp.qmi, P.Scxl,
+                        // reciprocals of the FP32 form's map
+                        1.0 / P.Scxl, 1.0 / (beta0 * gambet), 1.0 / (beta0 * P.Scxl), 1.0 / qm0};
   std::memcpy(op.c, c, sizeof(c));
   return op;
 }
@@ -858,7 +862,7 @@ void bend_sector_op(const Phys& P, const BendState& bs, double len, const Specie
   const double gambet = beta0 / std::sqrt(1.0 - beta0 * beta0);
   const double gam2 = 1.0 / (1.0 - beta0 * beta0);
   const double gam0 = std::sqrt(gam2);
-  const double c[33] = {ct,
+  const double c[37] = {ct,
                         rho * st,
                         R16,
                         -st / rho,
@@ -890,7 +894,11 @@ void bend_sector_op(const Phys& P, const BendState& bs, double len, const Specie
                         gam0,
                         bs.qm0,
                         sp.qmi,
-                        P.Scxl};
+                        P.Scxl,
+                        1.0 / P.Scxl,  // reciprocals of the FP32 form's map
+                        1.0 / (beta0 * gambet),
+                        1.0 / (beta0 * P.Scxl),
+                        1.0 / bs.qm0};
   std::memcpy(op.c, c, sizeof(c));
   push_op(prog, op);
 }
@@ -1293,6 +1301,7 @@ int drift2_op(const Phys& P, double tau, double refptcl[6], MapProgram& prog) {
   const double gamma0 = -refptcl[5];
   const double beta0 = std::sqrt(1.0 - 1.0 / gamma0 / gamma0);
   op.c[0] = gamma0; op.c[1] = beta0; op.c[2] = P.Scxl; op.c[3] = tau;
+  op.c[4] = 0.5 * tau / P.Scxl; op.c[5] = 1.0 / beta0;  // the FP32 form's map
   refptcl[4] = refptcl[4] + 0.5 * tau / (P.Scxl * beta0);
   return push_op(prog, op);
 }
