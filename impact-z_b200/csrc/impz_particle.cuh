@@ -549,6 +549,13 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
   return v;
 }
 
+// m = max(m, x) and m = min(m, x) for a bound m that is never NaN; like fmax
+// and fmin they pass over a NaN x, but a compare and a select do.  The pass
+// has 17 of them per particle: 248 us with fmax and fmin at 4e6 particles
+// (light pass, FP32 form), 234 with these.
+__device__ __forceinline__ void raise_to(double& m, double x) { m = x > m ? x : m; }
+__device__ __forceinline__ void lower_to(double& m, double x) { m = x < m ? x : m; }
+
 // the 37 sums of diagnostic1_Output (Output.f90:133-196), in tmplc order
 __device__ __forceinline__ void moment_accumulate(double* s, const Particle& p) {
   const double x = p.x, px = p.px, y = p.y, py = p.py, z = p.ph, pz = p.pt;
@@ -743,15 +750,15 @@ __device__ __forceinline__ void warp_moments(double* tile, const Contrib (&c)[U]
   double* row = tile + lane * IMPZ_MSUMS;
 #pragma unroll
   for (int v = 0; v < IMPZ_MSUMS; v++) {
-    double s = 0.0;
+    double s = moment_value(c[0], v);
 #pragma unroll
-    for (int u = 0; u < U; u++) s = s + moment_value(c[u], v);
+    for (int u = 1; u < U; u++) s = s + moment_value(c[u], v);
     row[v] = s;
   }
 #pragma unroll
   for (int u = 0; u < U; u++)
 #pragma unroll
-    for (int v = 0; v < 7; v++) mx[v] = fmax(mx[v], moment_value(c[u], 37 + v));
+    for (int v = 0; v < 7; v++) raise_to(mx[v], moment_value(c[u], 37 + v));
   __syncwarp();
   double s0 = 0.0, s1 = 0.0;
 #pragma unroll 8
@@ -1213,12 +1220,12 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
         if (SP && a.sp_cnt) atomicAdd(&s_spc[spi[u]], 1);
         if (rng) {
           const TFrame t = to_tframe(p[u], gam_n, rad_n, xl);
-          rmn[0] = fmin(rmn[0], fmin(t.tmpx, t.xt));
-          rmx[0] = fmax(rmx[0], fmax(t.tmpx, t.xt));
-          rmn[1] = fmin(rmn[1], fmin(t.tmpy, t.yt));
-          rmx[1] = fmax(rmx[1], fmax(t.tmpy, t.yt));
-          rmn[2] = fmin(rmn[2], t.zt);
-          rmx[2] = fmax(rmx[2], t.zt);
+          lower_to(rmn[0], t.tmpx); lower_to(rmn[0], t.xt);
+          raise_to(rmx[0], t.tmpx); raise_to(rmx[0], t.xt);
+          lower_to(rmn[1], t.tmpy); lower_to(rmn[1], t.yt);
+          raise_to(rmx[1], t.tmpy); raise_to(rmx[1], t.yt);
+          lower_to(rmn[2], t.zt);
+          raise_to(rmx[2], t.zt);
           nlive += t.lost ? 0 : 1;
           if (a.tframe) {  // stored as conv1st leaves Pts1 (stored_tframe)
             p[u].x = t.xt;
