@@ -689,6 +689,7 @@ int half_map_ops(const Phys& P, const impz_elem_t& e, double zedge, double z, do
     const double beta0 = gambet0 / gam0;
     MapOp op = blank(MAP_DRIFT);
     op.c[0] = gam0; op.c[1] = beta0; op.c[2] = tau; op.c[3] = Scxl;
+    op.c[4] = 1.0 / beta0; op.c[5] = tau / Scxl;
     refptcl[4] = refptcl[4] + tau / (Scxl * beta0);
     return push_op(prog, op);
   }

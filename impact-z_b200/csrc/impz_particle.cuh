@@ -48,17 +48,20 @@ struct Particle {
 // ---------------------------------------------------------------------
 // transfer maps; each follows the cited reference loop body
 __device__ __forceinline__ void map_drift(Particle& p, const volatile double* c) {
-  // BeamBunch.f90:286-295; c = {gam0, beta0, tau, Scxl}
-  const double gam0 = c[0], beta0 = c[1], tau = c[2], Scxl = c[3];
+  // BeamBunch.f90:286-295; c = {gam0, beta0, tau, Scxl, 1/beta0, tau/Scxl}
+  const double gam0 = c[0];
   double d = p.pt - gam0;
 #if IMPZ_FASTMATH
-  // one reciprocal square root instead of seven divisions
+  // one reciprocal square root instead of the divisions; the host's quotients
+  // c[4] and c[5] (the coefficients are re-read per particle, so a quotient
+  // of them here was a division per particle)
   const double rt = rsqrt(((d * d - 1.0) - p.px * p.px) - p.py * p.py);
-  const double ts = tau / Scxl;
+  const double ts = c[5];
   p.x = p.x + p.px * ts * rt;
   p.y = p.y + p.py * ts * rt;
-  p.ph = p.ph - (1.0 / beta0 + d * rt) * ts;
+  p.ph = p.ph - (c[4] + d * rt) * ts;
 #else
+  const double beta0 = c[1], tau = c[2], Scxl = c[3];
   double tmph = sqrt(((d * d - 1.0) - p.px * p.px) - p.py * p.py);
   p.x = p.x + ((p.px * tau) / tmph) / Scxl;
   p.y = p.y + ((p.py * tau) / tmph) / Scxl;
@@ -516,6 +519,23 @@ __device__ __forceinline__ Cell cic_cell(double x, double y, double z, const GT&
   c.cd = __dmul_rn(__dadd_rn(__dsub_rn(g.range[2], y), __dmul_rn((double)c.jx, g.h[1])), g.hi[1]);
   c.kx = (int)__dadd_rn(__dmul_rn(__dsub_rn(z, g.range[4]), g.hi[2]), 1.0);
   c.ef = __dmul_rn(__dadd_rn(__dsub_rn(g.range[4], z), __dmul_rn((double)c.kx, g.h[2])), g.hi[2]);
+  return c;
+}
+
+// The same cell and weights for the gather of the FP32 form, whose cell no
+// other kernel has to agree on: ab = ix - (x - xmin)/hx.
+template <typename GT>
+__device__ __forceinline__ Cell cic_cell_fast(double x, double y, double z, const GT& g) {
+  Cell c;
+  const double tx = (x - g.range[0]) * g.hi[0];
+  const double ty = (y - g.range[2]) * g.hi[1];
+  const double tz = (z - g.range[4]) * g.hi[2];
+  c.ix = (int)(tx + 1.0);
+  c.jx = (int)(ty + 1.0);
+  c.kx = (int)(tz + 1.0);
+  c.ab = (double)c.ix - tx;
+  c.cd = (double)c.jx - ty;
+  c.ef = (double)c.kx - tz;
   return c;
 }
 
@@ -1066,6 +1086,9 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
   const bool rng = pre && sp->range_next;
   const double gam = sp->gam, rad = sp->rad;
   const double gam_n = sp[1].gam, rad_n = sp[1].rad;
+#if IMPZ_FASTMATH
+  const double xkg = -xk / gam;
+#endif
   double txy = 0.0, tt = 0.0;
   if (kick) {
     double xycon, tcon;
@@ -1139,8 +1162,6 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
           const double rcp = t.rcp;
 #if IMPZ_FASTMATH
           const double rb = rsqrt(t.tmpbet);  // 1/betai
-          const double betai = t.tmpbet * rb;
-          const double xkg = -xk / gam;
           const double ph1 = t.zt * xkg * rb;
 #else
           const double betai = sqrt(t.tmpbet);
@@ -1149,9 +1170,16 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
           const double x1 = t.xt * xk + p[u].px * ph1 * rcp;
           const double y1 = t.yt * xk + p[u].py * ph1 * rcp;
           const double xg = x1 * xl, yg = y1 * xl;
+          // scatter1 (BeamBunch.f90:2121-2177); indices clamped into the grid.
+          // Its return to the phase (and the phase's way to z before it)
+          // undoes cvbkforth1st's step exactly, so the FP32 form keeps ph1,
+          // x1, y1 and z_t instead of multiplying back and forth.
+#if IMPZ_FASTMATH
+          Cell cg = cic_cell_fast(xg, yg, t.zt, g);
+#else
           const double zg = -(gam * betai * ph1 * xl);
-          // scatter1 (BeamBunch.f90:2121-2177); indices clamped into the grid
           Cell cg = cic_cell(xg, yg, zg, g);
+#endif
           if (!cell_inside(cg, nx, ny, nz)) {
             err |= DERR_OUTSIDE;
             cg.ix = min(max(cg.ix, 1), nx - 1);
@@ -1166,11 +1194,13 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
             ez = ez * a.efield_scale;
           }
           const double exn = ex * gam, eyn = ey * gam, ezn = ez;
+#if IMPZ_FASTMATH
+          p[u].x = x1;
+          p[u].y = y1;
+          p[u].ph = ph1;
+#else
           p[u].x = xg * xk;
           p[u].y = yg * xk;
-#if IMPZ_FASTMATH
-          p[u].ph = zg * xkg * rb;
-#else
           p[u].ph = zg * xk / (-(gam * betai));
 #endif
           if (!LIGHT && sp->lorentz) {
