@@ -32,9 +32,6 @@ inline cudaError_t launch_pdl(void (*kernel)(KP...), dim3 grid, dim3 block, size
 #ifndef IMPZ_ADV_U
 #define IMPZ_ADV_U 2
 #endif
-#ifndef IMPZ_ADV_PREFETCH
-#define IMPZ_ADV_PREFETCH 0
-#endif
 #ifndef IMPZ_ADV_MINB
 #define IMPZ_ADV_MINB 2
 #endif

@@ -55,11 +55,12 @@ __device__ __forceinline__ void map_drift(Particle& p, const volatile double* c)
   // one reciprocal square root instead of the divisions; the host's quotients
   // c[4] and c[5] (the coefficients are re-read per particle, so a quotient
   // of them here was a division per particle)
-  const double rt = rsqrt(((d * d - 1.0) - p.px * p.px) - p.py * p.py);
-  const double ts = c[5];
-  p.x = p.x + p.px * ts * rt;
-  p.y = p.y + p.py * ts * rt;
-  p.ph = p.ph - (c[4] + d * rt) * ts;
+  const double rt =
+      rsqrt(__fma_rn(-p.py, p.py, __fma_rn(-p.px, p.px, __fma_rn(d, d, -1.0))));
+  const double ts = c[5], tr = __dmul_rn(ts, rt);
+  p.x = __fma_rn(p.px, tr, p.x);
+  p.y = __fma_rn(p.py, tr, p.y);
+  p.ph = __fma_rn(-__fma_rn(d, rt, c[4]), ts, p.ph);
 #else
   const double beta0 = c[1], tau = c[2], Scxl = c[3];
   double tmph = sqrt(((d * d - 1.0) - p.px * p.px) - p.py * p.py);
@@ -397,32 +398,38 @@ __device__ __forceinline__ void map_sector(Particle& p, const volatile double* c
 // drift/quadrupole lattices); the host picks that instantiation when every
 // step of a run qualifies, which keeps the other map kinds' code and
 // registers out of the particle pass.
-// qmi: the particle's Pts1(7), read by the K-map and the bend maps.
-template <bool LIGHT>
-__device__ __forceinline__ void apply_program(Particle& p, const volatile MapProgram& prog,
-                                              const double qmi) {
+// qmi: the particles' Pts1(7), read by the K-map and the bend maps.
+// Every op is applied to the thread's U particles in turn, so that a
+// coefficient's load serves them all and their arithmetic interleaves.
+template <bool LIGHT, int U>
+__device__ __forceinline__ void apply_program(Particle (&p)[U], const volatile MapProgram& prog,
+                                              const double (&qmi)[U]) {
   const int nops = prog.nops;
+#define IMPZ_EACH(map)          \
+  _Pragma("unroll") for (int u = 0; u < U; u++) { map; }
   for (int o = 0; o < nops; o++) {
     const volatile MapOp& op = prog.ops[o];
+    const int kind = op.kind;
     if (LIGHT) {
-      if (op.kind == MAP_DRIFT) map_drift(p, op.c);
-      else if (op.kind == MAP_XM2) map_xm2(p, op.c);
+      if (kind == MAP_DRIFT) { IMPZ_EACH(map_drift(p[u], op.c)) }
+      else if (kind == MAP_XM2) { IMPZ_EACH(map_xm2(p[u], op.c)) }
       continue;
     }
-    switch (op.kind) {
-      case MAP_DRIFT: map_drift(p, op.c); break;
-      case MAP_XM6: map_xm6(p, op.c, op.flags, op.iparam); break;
-      case MAP_KQUAD: map_kquad(p, op.c, qmi); break;
-      case MAP_IDEALRF: map_idealrf(p, op.c, op.flags, op.iparam); break;
-      case MAP_FPOL: map_pole<false>(p, op.c, qmi); break;
-      case MAP_BPOL: map_pole<true>(p, op.c, qmi); break;
-      case MAP_SECTOR: map_sector(p, op.c, qmi); break;
-      case MAP_XM2: map_xm2(p, op.c); break;
-      case MAP_UNDUL: map_undul(p, op.c); break;
-      case MAP_DRIFT2: map_drift2(p, op.c); break;
+    switch (kind) {
+      case MAP_DRIFT: IMPZ_EACH(map_drift(p[u], op.c)) break;
+      case MAP_XM6: IMPZ_EACH(map_xm6(p[u], op.c, op.flags, op.iparam)) break;
+      case MAP_KQUAD: IMPZ_EACH(map_kquad(p[u], op.c, qmi[u])) break;
+      case MAP_IDEALRF: IMPZ_EACH(map_idealrf(p[u], op.c, op.flags, op.iparam)) break;
+      case MAP_FPOL: IMPZ_EACH(map_pole<false>(p[u], op.c, qmi[u])) break;
+      case MAP_BPOL: IMPZ_EACH(map_pole<true>(p[u], op.c, qmi[u])) break;
+      case MAP_SECTOR: IMPZ_EACH(map_sector(p[u], op.c, qmi[u])) break;
+      case MAP_XM2: IMPZ_EACH(map_xm2(p[u], op.c)) break;
+      case MAP_UNDUL: IMPZ_EACH(map_undul(p[u], op.c)) break;
+      case MAP_DRIFT2: IMPZ_EACH(map_drift2(p[u], op.c)) break;
       default: break;
     }
   }
+#undef IMPZ_EACH
 }
 
 // Copies a step's programs into shared memory (whole block).
@@ -523,19 +530,22 @@ __device__ __forceinline__ Cell cic_cell(double x, double y, double z, const GT&
 }
 
 // The same cell and weights for the gather of the FP32 form, whose cell no
-// other kernel has to agree on: ab = ix - (x - xmin)/hx.
+// other kernel has to agree on: ab = ix - (x - xmin)/hx.  Rounded explicitly
+// all the same: a bunch alone and in a packed launch run two instantiations
+// of the pass, and where the compiler contracted them differently a last bit
+// here became an FP32 weight's.
 template <typename GT>
 __device__ __forceinline__ Cell cic_cell_fast(double x, double y, double z, const GT& g) {
   Cell c;
-  const double tx = (x - g.range[0]) * g.hi[0];
-  const double ty = (y - g.range[2]) * g.hi[1];
-  const double tz = (z - g.range[4]) * g.hi[2];
-  c.ix = (int)(tx + 1.0);
-  c.jx = (int)(ty + 1.0);
-  c.kx = (int)(tz + 1.0);
-  c.ab = (double)c.ix - tx;
-  c.cd = (double)c.jx - ty;
-  c.ef = (double)c.kx - tz;
+  const double tx = __dmul_rn(__dsub_rn(x, g.range[0]), g.hi[0]);
+  const double ty = __dmul_rn(__dsub_rn(y, g.range[2]), g.hi[1]);
+  const double tz = __dmul_rn(__dsub_rn(z, g.range[4]), g.hi[2]);
+  c.ix = (int)__dadd_rn(tx, 1.0);
+  c.jx = (int)__dadd_rn(ty, 1.0);
+  c.kx = (int)__dadd_rn(tz, 1.0);
+  c.ab = __dsub_rn((double)c.ix, tx);
+  c.cd = __dsub_rn((double)c.jx, ty);
+  c.ef = __dsub_rn((double)c.kx, tz);
   return c;
 }
 
@@ -1108,148 +1118,144 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
 
   const long long stride = (long long)vgx * BLOCK * U;
   const long long nround = (n + stride - 1) / stride * stride;
-  // the next pass's particles are loaded while this pass computes (each
-  // thread reads its own slots only; in-place launches write slot i back)
-  Particle nxt[U];
-  auto fetch = [&](long long ib) {
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const long long i = ib + (long long)u * BLOCK;
-      if (i < n) {
-        nxt[u].x = a.in[0][i]; nxt[u].px = a.in[1][i]; nxt[u].y = a.in[2][i];
-        nxt[u].py = a.in[3][i]; nxt[u].ph = a.in[4][i]; nxt[u].pt = a.in[5][i];
-      } else {
-        nxt[u].x = 0; nxt[u].px = 0; nxt[u].y = 0; nxt[u].py = 0; nxt[u].ph = 0; nxt[u].pt = 0;
-      }
-    }
-  };
-#if IMPZ_ADV_PREFETCH
-  fetch((long long)vbx * BLOCK * U + threadIdx.x);
-#endif
-  for (long long i0 = (long long)vbx * BLOCK * U + threadIdx.x; i0 < nround;
-       i0 += stride) {
+  // Every stage runs for the thread's U particles without a branch on the
+  // particle, so that their dependent FP64 chains interleave; what a lost or
+  // absent particle computes (zeros, or a lost mark's NaN; its cell indices
+  // are clamped like any other's) is dropped where something is kept.  With
+  // a particle's chain behind its own branch the pass of 4e6 particles took
+  // 227 us (220 so), that of 2e7 electrons mostly in sector bends 1502
+  // (1349).  Reciprocals and square roots of our own without the library
+  // functions' special-case branches were slower (238).
+  for (long long i0 = (long long)vbx * BLOCK * U + threadIdx.x; i0 < nround; i0 += stride) {
     Particle p[U];
     bool keep[U];
     int key[U];  // deposit cell (a grid holds at most 64 x 64 x 4096 nodes)
     int spi[U];  // species index (0 for a single-species bunch)
-#if !IMPZ_ADV_PREFETCH
-    fetch(i0);
-#endif
+    double qmi[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const long long i = i0 + (long long)u * BLOCK;
       keep[u] = i < n;
       key[u] = 0;
-      p[u] = nxt[u];
+      p[u].x = p[u].px = p[u].y = p[u].py = p[u].ph = p[u].pt = 0.0;
+      if (keep[u]) {
+        p[u].x = a.in[0][i]; p[u].px = a.in[1][i]; p[u].y = a.in[2][i];
+        p[u].py = a.in[3][i]; p[u].ph = a.in[4][i]; p[u].pt = a.in[5][i];
+      }
       spi[u] = (species && keep[u]) ? (int)a.sp_in[i] : 0;
+      qmi[u] = species ? __ldg(a.sp_qm + spi[u]) : a.k.qmi;
     }
-#if IMPZ_ADV_PREFETCH
-    if (i0 + stride < nround) fetch(i0 + stride);
-#endif
     Contrib c[U];
+    if (kick) {
+      if (!a.tframe) {  // hold them as the whole-lattice runner stores them
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      if (keep[u] && kick) {
-        const TFrame t = a.tframe ? stored_tframe(p[u], gam) : to_tframe(p[u], gam, rad, xl);
-        if (t.lost) {
-          keep[u] = false;
-        } else {
-          Cell cd = cic_cell(t.xt, t.yt, t.zt, g);
-          key[u] = cell_inside(cd, nx, ny, nz) ? cell_key(cd.ix - 1, cd.jx - 1, cd.kx - 1, nx, ny)
-                                                : (int)G;
-          // cvbkforth1st (BeamBunch.f90:1681-1699); betai reuses conv1st's
-          // tmpbet, the same expression of the same operands
-          const double rcp = t.rcp;
-#if IMPZ_FASTMATH
-          const double rb = rsqrt(t.tmpbet);  // 1/betai
-          const double ph1 = t.zt * xkg * rb;
-#else
-          const double betai = sqrt(t.tmpbet);
-          const double ph1 = t.zt * xk / (-(gam * betai));
-#endif
-          const double x1 = t.xt * xk + p[u].px * ph1 * rcp;
-          const double y1 = t.yt * xk + p[u].py * ph1 * rcp;
-          const double xg = x1 * xl, yg = y1 * xl;
-          // scatter1 (BeamBunch.f90:2121-2177); indices clamped into the grid.
-          // Its return to the phase (and the phase's way to z before it)
-          // undoes cvbkforth1st's step exactly, so the FP32 form keeps ph1,
-          // x1, y1 and z_t instead of multiplying back and forth.
-#if IMPZ_FASTMATH
-          Cell cg = cic_cell_fast(xg, yg, t.zt, g);
-#else
-          const double zg = -(gam * betai * ph1 * xl);
-          Cell cg = cic_cell(xg, yg, zg, g);
-#endif
-          if (!cell_inside(cg, nx, ny, nz)) {
-            err |= DERR_OUTSIDE;
-            cg.ix = min(max(cg.ix, 1), nx - 1);
-            cg.jx = min(max(cg.jx, 1), ny - 1);
-            cg.kx = min(max(cg.kx, 1), nz - 1);
-          }
-          double ex, ey, ez;
-          gather_e<F32>(a.efield, cg, nx, ny, ex, ey, ez);
-          if (F32) {
-            ex = ex * a.efield_scale;
-            ey = ey * a.efield_scale;
-            ez = ez * a.efield_scale;
-          }
-          const double exn = ex * gam, eyn = ey * gam, ezn = ez;
-#if IMPZ_FASTMATH
-          p[u].x = x1;
-          p[u].y = y1;
-          p[u].ph = ph1;
-#else
-          p[u].x = xg * xk;
-          p[u].y = yg * xk;
-          p[u].ph = zg * xk / (-(gam * betai));
-#endif
-          if (!LIGHT && sp->lorentz) {
-            // scatter2_BeamBunch (BeamBunch.f90:2766-3065): the same way back
-            // to the z frame, then the implicit Lorentz update
-            // scatter2wake: the wake's planes kx, kx+1 weighted by the
-            // gather cell's ef (BeamBunch.f90:5634-5636)
-            double wx = 0.0, wy = 0.0, wz = 0.0;
-            if ((sp->csr || sp->wake) && a.wake_raw) {
-              const double* w = a.wake_raw + (cg.kx - 1);
-              wx = w[0] * cg.ef + w[1] * (1.0 - cg.ef);
-              wy = w[nz] * cg.ef + w[nz + 1] * (1.0 - cg.ef);
-              wz = w[2 * nz] * cg.ef + w[2 * nz + 1] * (1.0 - cg.ef);
-            }
-            lorentz_kick(p[u], exn, eyn, ezn, gam, sp, a.k, wx, wy, wz, a.lz_data,
-                         species ? __ldg(a.sp_qm + spi[u]) : a.k.qmi);
-          } else {
-            p[u].px = p[u].px + txy * exn;
-            p[u].py = p[u].py + txy * eyn;
-            p[u].pt = p[u].pt - tt * ezn;
-          }
+        for (int u = 0; u < U; u++) {
+          const TFrame t = to_tframe(p[u], gam, rad, xl);
+          p[u].x = t.xt;
+          p[u].y = t.yt;
+          p[u].ph = t.lost ? lost_mark() : t.zt;
         }
       }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const TFrame t = stored_tframe(p[u], gam);
+        keep[u] = keep[u] && !t.lost;
+        const Cell cd = cic_cell(t.xt, t.yt, t.zt, g);
+        key[u] = cell_inside(cd, nx, ny, nz) ? cell_key(cd.ix - 1, cd.jx - 1, cd.kx - 1, nx, ny)
+                                              : (int)G;
+        // cvbkforth1st (BeamBunch.f90:1681-1699); betai reuses conv1st's
+        // tmpbet, the same expression of the same operands
+        const double rcp = t.rcp;
+#if IMPZ_FASTMATH
+        const double ph1 = __dmul_rn(__dmul_rn(t.zt, xkg), rsqrt(t.tmpbet));
+        const double phr = __dmul_rn(ph1, rcp);
+        const double x1 = __fma_rn(p[u].px, phr, __dmul_rn(t.xt, xk));
+        const double y1 = __fma_rn(p[u].py, phr, __dmul_rn(t.yt, xk));
+        const double xg = __dmul_rn(x1, xl), yg = __dmul_rn(y1, xl);
+#else
+        const double betai = sqrt(t.tmpbet);
+        const double ph1 = t.zt * xk / (-(gam * betai));
+        const double x1 = t.xt * xk + p[u].px * ph1 * rcp;
+        const double y1 = t.yt * xk + p[u].py * ph1 * rcp;
+        const double xg = x1 * xl, yg = y1 * xl;
+#endif
+        // scatter1 (BeamBunch.f90:2121-2177); indices clamped into the grid.
+        // Its return to the phase (and the phase's way to z before it)
+        // undoes cvbkforth1st's step exactly, so the FP32 form keeps ph1,
+        // x1, y1 and z_t instead of multiplying back and forth.
+#if IMPZ_FASTMATH
+        Cell cg = cic_cell_fast(xg, yg, t.zt, g);
+#else
+        const double zg = -(gam * betai * ph1 * xl);
+        Cell cg = cic_cell(xg, yg, zg, g);
+#endif
+        if (keep[u] && !cell_inside(cg, nx, ny, nz)) err |= DERR_OUTSIDE;
+        cg.ix = min(max(cg.ix, 1), nx - 1);
+        cg.jx = min(max(cg.jx, 1), ny - 1);
+        cg.kx = min(max(cg.kx, 1), nz - 1);
+        double ex, ey, ez;
+        gather_e<F32>(a.efield, cg, nx, ny, ex, ey, ez);
+        if (F32) {
+          ex = ex * a.efield_scale;
+          ey = ey * a.efield_scale;
+          ez = ez * a.efield_scale;
+        }
+        const double exn = ex * gam, eyn = ey * gam, ezn = ez;
+#if IMPZ_FASTMATH
+        p[u].x = x1;
+        p[u].y = y1;
+        p[u].ph = ph1;
+#else
+        p[u].x = xg * xk;
+        p[u].y = yg * xk;
+        p[u].ph = zg * xk / (-(gam * betai));
+#endif
+        if (!LIGHT && sp->lorentz) {
+          // scatter2_BeamBunch (BeamBunch.f90:2766-3065): the same way back
+          // to the z frame, then the implicit Lorentz update
+          // scatter2wake: the wake's planes kx, kx+1 weighted by the
+          // gather cell's ef (BeamBunch.f90:5634-5636)
+          double wx = 0.0, wy = 0.0, wz = 0.0;
+          if ((sp->csr || sp->wake) && a.wake_raw) {
+            const double* w = a.wake_raw + (cg.kx - 1);
+            wx = w[0] * cg.ef + w[1] * (1.0 - cg.ef);
+            wy = w[nz] * cg.ef + w[nz + 1] * (1.0 - cg.ef);
+            wz = w[2 * nz] * cg.ef + w[2 * nz + 1] * (1.0 - cg.ef);
+          }
+          lorentz_kick(p[u], exn, eyn, ezn, gam, sp, a.k, wx, wy, wz, a.lz_data, qmi[u]);
+        } else {
+          p[u].px = p[u].px + txy * exn;
+          p[u].py = p[u].py + txy * eyn;
+          p[u].pt = p[u].pt - tt * ezn;
+        }
+      }
+    } else if (!LIGHT && post && sp->lorentz) {
       // a Lorentz-integrator step without space charge: scatter20's kick by
       // the element's field alone, on the stored coordinates
       // (BeamBunch.f90:3075-3531)
-      if (!LIGHT && keep[u] && !kick && post && sp->lorentz)
-        lorentz_kick(p[u], 0.0, 0.0, 0.0, gam, sp, a.k, 0.0, 0.0, 0.0, a.lz_data,
-                     species ? __ldg(a.sp_qm + spi[u]) : a.k.qmi);
-      if (keep[u] && post)
-        apply_program<LIGHT>(p[u], progs[0], species ? __ldg(a.sp_qm + spi[u]) : a.k.qmi);
-      if (keep[u]) {
-        c[u].x = p[u].x; c[u].px = p[u].px; c[u].y = p[u].y;
-        c[u].py = p[u].py; c[u].z = p[u].ph; c[u].pz = p[u].pt;
-      } else {
-        c[u].x = 0; c[u].px = 0; c[u].y = 0; c[u].py = 0; c[u].z = 0; c[u].pz = 0;
-      }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        lorentz_kick(p[u], 0.0, 0.0, 0.0, gam, sp, a.k, 0.0, 0.0, 0.0, a.lz_data, qmi[u]);
     }
-    if (mom) warp_moments<U>(mtile_dyn + wid * 32 * IMPZ_MSUMS, c, lane, macc0, macc1, mmax);
+    if (post) apply_program<LIGHT, U>(p, progs[0], qmi);
+    if (mom) {
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        c[u].x = keep[u] ? p[u].x : 0.0; c[u].px = keep[u] ? p[u].px : 0.0;
+        c[u].y = keep[u] ? p[u].y : 0.0; c[u].py = keep[u] ? p[u].py : 0.0;
+        c[u].z = keep[u] ? p[u].ph : 0.0; c[u].pz = keep[u] ? p[u].pt : 0.0;
+      }
+      warp_moments<U>(mtile_dyn + wid * 32 * IMPZ_MSUMS, c, lane, macc0, macc1, mmax);
+    }
+    if (pre) apply_program<LIGHT, U>(p, progs[1], qmi);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      if (keep[u]) {
-        if (pre)
-          apply_program<LIGHT>(p[u], progs[1], species ? __ldg(a.sp_qm + spi[u]) : a.k.qmi);
-        if (!finite6(p[u])) err |= DERR_NONFINITE;
-        nkept++;
-        if (SP && a.sp_cnt) atomicAdd(&s_spc[spi[u]], 1);
-        if (rng) {
-          const TFrame t = to_tframe(p[u], gam_n, rad_n, xl);
+      if (keep[u] && !finite6(p[u])) err |= DERR_NONFINITE;
+      nkept += keep[u] ? 1 : 0;
+      if (SP && a.sp_cnt && keep[u]) atomicAdd(&s_spc[spi[u]], 1);
+      if (rng) {
+        const TFrame t = to_tframe(p[u], gam_n, rad_n, xl);
+        if (keep[u]) {
           lower_to(rmn[0], t.tmpx); lower_to(rmn[0], t.xt);
           raise_to(rmx[0], t.tmpx); raise_to(rmx[0], t.xt);
           lower_to(rmn[1], t.tmpy); lower_to(rmn[1], t.yt);
@@ -1257,11 +1263,11 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
           lower_to(rmn[2], t.zt);
           raise_to(rmx[2], t.zt);
           nlive += t.lost ? 0 : 1;
-          if (a.tframe) {  // stored as conv1st leaves Pts1 (stored_tframe)
-            p[u].x = t.xt;
-            p[u].y = t.yt;
-            p[u].ph = t.lost ? lost_mark() : t.zt;
-          }
+        }
+        if (a.tframe) {  // stored as conv1st leaves Pts1 (stored_tframe)
+          p[u].x = t.xt;
+          p[u].y = t.yt;
+          p[u].ph = t.lost ? lost_mark() : t.zt;
         }
       }
       // destination slot
