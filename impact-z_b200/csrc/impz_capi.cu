@@ -234,10 +234,29 @@ __global__ void k_soa_to_aos(double* __restrict__ aos, long long n, long long i0
   }
 }
 
-__global__ void k_e4_to_grid(const void* e4, int f32, long long G, int c, double* out) {
+// component c of the node field; the FP32 form's is per unit charge weight
+__global__ void k_e4_to_grid(const void* e4, int f32, long long G, int c, double weight,
+                             double* out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < G;
        i += (long long)gridDim.x * blockDim.x)
-    out[i] = f32 ? (double)((const float*)e4)[4 * i + c] : ((const double*)e4)[4 * i + c];
+    out[i] = f32 ? (double)((const float*)e4)[4 * i + c] * weight : ((const double*)e4)[4 * i + c];
+}
+
+// What impz_deposit returns, x fastest: the charge grid in Coulomb (q: the
+// value of a quantum) and the per-cell counts, which are kept in sort-key
+// order (cell_key, impz_particle.cuh).  Either output may be null.
+__global__ void k_charge_out(const unsigned long long* __restrict__ rho,
+                             const int* __restrict__ counts, int nx, int ny, long long G, double q,
+                             double* chg, int* cnt) {
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < G;
+       e += (long long)gridDim.x * blockDim.x) {
+    if (chg) chg[e] = (double)(long long)rho[e] * q;
+    if (cnt) {
+      const int i = (int)(e % nx), j = (int)(e / nx % ny), k = (int)(e / ((long long)nx * ny));
+      const int brick = ((k >> 2) * (ny >> 2) + (j >> 2)) * (nx >> 2) + (i >> 2);
+      cnt[e] = counts[(brick << 6) | ((k & 3) << 4) | ((j & 3) << 2) | (i & 3)];
+    }
+  }
 }
 
 // per-block sums of cos(kz * phase) and sin(kz * phase) (bunching factor)
@@ -1439,37 +1458,26 @@ int impz_deposit(impz_bunch_t b, double* chgdens, int* counts) {
     ProfScope ps(b, IMPZ_PROF_DEPOSIT, 1);
     CK(launch_deposit(b, d));
   }
-  std::vector<int> keyed;
-  if (counts) {  // per-cell counts are kept in sort-key order (cell_key, impz_particle.cuh)
-    keyed.resize((size_t)b->G);
-    CK(cudaMemcpyAsync(keyed.data(), b->counts, b->G * sizeof(int), cudaMemcpyDeviceToHost,
-                       b->stream));
-  }
-  std::vector<long long> q;
-  if (chgdens) {
-    q.resize((size_t)b->G);
-    CK(cudaMemcpyAsync(q.data(), b->rho, b->G * sizeof(long long), cudaMemcpyDeviceToHost,
-                       b->stream));
+  // the grids go out through the (idle) spectrum, which holds at least 16 G
+  // bytes, converted and reordered on the device: the host's loops over the
+  // nodes and the scratch vectors cost more than the deposit itself
+  double* chg = chgdens ? (double*)b->spec : nullptr;
+  int* cnt = counts ? (int*)((double*)b->spec + b->G) : nullptr;
+  if (chg || cnt) {
+    k_charge_out<<<(int)std::min<long long>((b->G + 255) / 256, 1184), 256, 0, b->stream>>>(
+        b->rho, b->counts, b->nx, b->ny, b->G, b->weight * std::ldexp(1.0, -b->fixbits), chg, cnt);
+    CK(cudaGetLastError());
+    g_launches += 1;
   }
   {
     ProfScope ps(b, IMPZ_PROF_SCAN, 1);
     CK(exact::launch_scan(b->counts, b->cursor, b->bsum, b->G + 1, b->st, b->stream));
   }
+  if (cnt)
+    CK(cudaMemcpyAsync(counts, cnt, b->G * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+  if (chg)
+    CK(cudaMemcpyAsync(chgdens, chg, b->G * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   CK(cudaStreamSynchronize(b->stream));
-  if (counts) {
-    const int nx = b->nx, ny = b->ny, nz = b->nz;
-    for (int k = 0; k < nz; k++)
-      for (int j = 0; j < ny; j++)
-        for (int i = 0; i < nx; i++) {
-          const int brick = ((k >> 2) * (ny >> 2) + (j >> 2)) * (nx >> 2) + (i >> 2);
-          const int key = (brick << 6) | ((k & 3) << 4) | ((j & 3) << 2) | (i & 3);
-          counts[i + (size_t)nx * (j + (size_t)ny * k)] = keyed[(size_t)key];
-        }
-  }
-  if (chgdens) {
-    const double qs = b->weight * std::ldexp(1.0, -b->fixbits);
-    for (long long i = 0; i < b->G; i++) chgdens[i] = (double)q[(size_t)i] * qs;
-  }
   b->stage = ST_DEPOSITED;
   return IMPZ_OK;
 }
@@ -1508,14 +1516,13 @@ static int kick_field(impz_bunch_t b, double* egrid) {
     // one component at a time through the (now free) spectrum, >= 16 G bytes
     double* tmp = (double*)b->spec;
     for (int c = 0; c < 3; c++) {
-      k_e4_to_grid<<<1184, 256, 0, b->stream>>>(b->efield, b->f32() ? 1 : 0, b->G, c, tmp);
+      k_e4_to_grid<<<1184, 256, 0, b->stream>>>(b->efield, b->f32() ? 1 : 0, b->G, c, b->weight,
+                                                tmp);
       g_launches += 1;
       CK(cudaMemcpyAsync(egrid + c * b->G, tmp, b->G * sizeof(double), cudaMemcpyDeviceToHost,
                          b->stream));
     }
     CK(cudaStreamSynchronize(b->stream));
-    if (b->f32())
-      for (long long i = 0; i < 3 * b->G; i++) egrid[i] *= b->weight;
   }
   return IMPZ_OK;
 }
