@@ -366,8 +366,9 @@ class Bunch:
         return rng, ms
 
     def autotune(self, nsteps=8):
-        """Picks deposit and push blocks and the z convolution's lines per
-        block by timing this bunch; the bunch is left as it was."""
+        """Picks deposit and push blocks by timing this bunch; the bunch is
+        left as it was.  z_lines is always 0: the z convolution has one
+        shape per length."""
         out = np.zeros(4)
         _check(lib().impz_autotune(self.h, int(nsteps), _dp(out)), "impz_autotune")
         return {"deposit_blocks": int(out[0]), "push_blocks": int(out[1]),
@@ -386,11 +387,11 @@ class Bunch:
         _check(lib().impz_bunch_set_z(self.h, float(z)), "impz_bunch_set_z")
 
     def download(self):
-        pts = np.zeros((self.n0, 9))
+        pts = np.empty((self.n0, 9))
         n = ctypes.c_longlong()
         _check(lib().impz_bunch_download(self.h, _dp(pts), self.n0, ctypes.byref(n)),
                "impz_bunch_download")
-        return pts[: n.value].copy()
+        return pts if n.value == self.n0 else pts[: n.value].copy()
 
     # --- the per-step surface -------------------------------------------
     def map_half(self, e, zedge, z, tau, nst, ihlf):
