@@ -482,15 +482,16 @@ struct impz_bunch_s {
   double sc_gam = 0, sc_rad = 0;
   // last impz_run_async
   CompiledLattice lat;
-  bool run_light = false;  // every step of the run needs only the light particle pass
+  PassKind run_pass = PASS_FULL;  // the particle pass that carries every step of the run
   bool run_pending = false;
   size_t bytes = 0;
   // graphs of two space-charge steps, per start parity and particle pass
-  // (graph 2 parity + light), and the buffers and wake generation each holds
-  cudaGraphExec_t gexec[4] = {nullptr, nullptr, nullptr, nullptr};
-  const StepParams* g_steps[4] = {nullptr, nullptr, nullptr, nullptr};
-  const double* g_mom[4] = {nullptr, nullptr, nullptr, nullptr};
-  int g_wake[4] = {-1, -1, -1, -1};
+  // (graph 2 pass + parity), and the buffers and wake generation each holds
+  static constexpr int kGraphs = 6;
+  cudaGraphExec_t gexec[kGraphs] = {};
+  const StepParams* g_steps[kGraphs] = {};
+  const double* g_mom[kGraphs] = {};
+  int g_wake[kGraphs] = {-1, -1, -1, -1, -1, -1};
   // read-in wakefield (impz_wake_set): table [3][ntab], then the line sums
   // [3][nz] and the per-plane field [3][nz] in one allocation
   bool wk_on = false, wk_tr = false;
@@ -509,7 +510,7 @@ struct impz_bunch_s {
   // the last per-step kick, grown as needed
   double* lzd = nullptr;
   size_t lzd_cap = 0;
-  const double* g_lzd[4] = {nullptr, nullptr, nullptr, nullptr};  // the data the step graphs point to
+  const double* g_lzd[kGraphs] = {};  // the data the step graphs point to
   int run_next = 0;       // next step of the run in progress
   double run_z = 0;       // z and refptcl at the end of the run in progress
   double run_ref[6] = {0};
@@ -614,34 +615,40 @@ AdvanceArgs advance_args(impz_bunch_t b, const StepParams* table, int fixed, int
   return a;
 }
 
-// `light`: every program of the table holds only drifts and block-diagonal
-// maps, so the particle pass without the other map kinds can run it
-cudaError_t launch_adv(impz_bunch_t b, const AdvanceArgs& a, bool light) {
+cudaError_t launch_adv(impz_bunch_t b, const AdvanceArgs& a, PassKind pass) {
   ProfScope ps(b, IMPZ_PROF_PUSH, 1);
-  if (b->f32()) return fast::launch_advance(a, true, light, b->grid_adv, b->stream);
-  return exact::launch_advance(a, false, light, b->grid_adv, b->stream);
+  if (b->f32()) return fast::launch_advance(a, pass, b->grid_adv, b->stream);
+  return exact::launch_advance(a, pass, b->grid_adv, b->stream);
 }
 
-bool program_is_light(const MapProgram& prog) {
+// the particle pass that carries what both passes' steps need
+PassKind wider(PassKind x, PassKind y) {
+  if (x == PASS_FULL || y == PASS_FULL) return PASS_FULL;
+  return x == PASS_MAPS || y == PASS_MAPS ? PASS_MAPS : PASS_LIGHT;
+}
+
+PassKind program_pass(const MapProgram& prog) {
+  PassKind pass = PASS_LIGHT;
   for (int o = 0; o < prog.nops; o++) {
     const int k = prog.ops[o].kind;
-    if (k != MAP_DRIFT && k != MAP_XM2 && k != MAP_NONE) return false;
+    if (k == MAP_IDEALRF) return PASS_FULL;
+    if (k != MAP_DRIFT && k != MAP_XM2 && k != MAP_NONE) pass = PASS_MAPS;
   }
-  return true;
+  return pass;
 }
 
-// whether the light particle pass can run step sp: drifts and block-diagonal
-// maps, no Lorentz kick (in the full pass only).  Chosen step by step: the
-// full pass spills registers and takes 1.8 times as long, and a lattice's
-// bends, cavities or K-map quadrupoles are often a few steps among many drifts
-bool step_is_light(const StepParams& sp) {
-  return !sp.lorentz && program_is_light(sp.post) && program_is_light(sp.pre_next);
+// The smallest instantiation of the particle pass for step sp, chosen step by
+// step: a lattice's bends, cavities or K-map quadrupoles are often a few steps
+// among many drifts.
+PassKind step_pass(const StepParams& sp) {
+  if (sp.lorentz) return PASS_FULL;
+  return wider(program_pass(sp.post), program_pass(sp.pre_next));
 }
 
-bool table_is_light(const std::vector<StepParams>& steps) {
-  for (const StepParams& sp : steps)
-    if (!step_is_light(sp)) return false;
-  return true;
+PassKind table_pass(const std::vector<StepParams>& steps) {
+  PassKind pass = PASS_LIGHT;
+  for (const StepParams& sp : steps) pass = wider(pass, step_pass(sp));
+  return pass;
 }
 
 DepositArgs deposit_args(impz_bunch_t b, const StepParams* table, int fixed) {
@@ -926,7 +933,7 @@ int build_species(impz_bunch_t b, const double* pts, long long n) {
   // the step graphs hold the weight (field scale), q/m and the number of
   // species by value
   if (b->weight != wref || b->sp.qmi != qm[0] || b->nspecies != (int)qm.size())
-    for (int p = 0; p < 4; p++)
+    for (int p = 0; p < impz_bunch_s::kGraphs; p++)
       if (b->gexec[p]) {
         cudaGraphExecDestroy(b->gexec[p]);
         b->gexec[p] = nullptr;
@@ -987,7 +994,7 @@ void free_bunch(impz_bunch_t b) {
   if (b->wk_mem) cudaFree(b->wk_mem);
   if (b->lzd) cudaFree(b->lzd);
   for (cudaEvent_t e : b->ev_pool) cudaEventDestroy(e);
-  for (int p = 0; p < 4; p++)
+  for (int p = 0; p < impz_bunch_s::kGraphs; p++)
     if (b->gexec[p]) cudaGraphExecDestroy(b->gexec[p]);
   if (b->stream2) cudaStreamSynchronize(b->stream2);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -1136,8 +1143,8 @@ int impz_bunch_create(const double* pts, long long n, double current, double mas
                      cudaMemcpyHostToDevice));
   }
   b->grid_adv = (int)std::min<long long>((n + IMPZ_ADV_BLOCK - 1) / IMPZ_ADV_BLOCK,
-                                         (long long)(b->f32() ? fast::max_blocks_advance(true)
-                                                              : exact::max_blocks_advance(false)));
+                                         (long long)(b->f32() ? fast::max_blocks_advance()
+                                                              : exact::max_blocks_advance()));
   b->grid_adv = std::min(b->grid_adv, kMaxAdvGrid);
   b->grid_dep = (int)std::min<long long>(
       (n + (long long)IMPZ_DEP_BLOCK * IMPZ_DEP_PPT - 1) / ((long long)IMPZ_DEP_BLOCK * IMPZ_DEP_PPT),
@@ -1359,7 +1366,7 @@ static int run_fine_advance(impz_bunch_t b, const StepParams host[2], int kick, 
   int r = upload_fine(b, host);
   if (r) return r;
   AdvanceArgs a = advance_args(b, b->dfine, 0, kick, post, pre, b->mom_fine, 0);
-  CK(launch_adv(b, a, step_is_light(host[0])));
+  CK(launch_adv(b, a, step_pass(host[0])));
   if (kick) b->parity ^= 1;
   if (rec) {
     CK(cudaMemcpyAsync(rec, b->mom_fine, IMPZ_MOMREC * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1725,13 +1732,13 @@ int impz_bunch_upload(impz_bunch_t b, const double* pts, long long n, double cur
 
 // ---- whole-lattice runner --------------------------------------------
 // One step s (read from DevState::step on the device) as direct launches.
-static int launch_step(impz_bunch_t b, bool sc, bool light) {
+static int launch_step(impz_bunch_t b, bool sc, PassKind pass) {
   if (sc) {
     int r = field_step(b, b->dsteps, -1);
     if (r) return r;
   }
   AdvanceArgs a = advance_args(b, b->dsteps, -1, sc ? 1 : 0, 1, 1, b->mom_out, 0);
-  CK(launch_adv(b, a, light));
+  CK(launch_adv(b, a, pass));
   if (sc) b->parity ^= 1;
   return IMPZ_OK;
 }
@@ -1782,8 +1789,8 @@ static int wake_key(impz_bunch_t b) { return 2 * b->wk_gen + (b->run_wake ? 1 : 
 // Two space-charge steps captured as one CUDA graph (parity returns to its
 // start value), cached per start parity and particle pass and re-captured
 // when the step table or the record buffer move.
-static int graph_pair(impz_bunch_t b, bool light) {
-  const int p = b->parity, k = 2 * p + (light ? 1 : 0);
+static int graph_pair(impz_bunch_t b, PassKind pass) {
+  const int p = b->parity, k = 2 * (int)pass + p;
   if (b->gexec[k] && (b->g_steps[k] != b->dsteps || b->g_mom[k] != b->mom_out ||
                       b->g_wake[k] != wake_key(b) || b->g_lzd[k] != b->lzd)) {
     cudaGraphExecDestroy(b->gexec[k]);
@@ -1793,8 +1800,8 @@ static int graph_pair(impz_bunch_t b, bool light) {
     cudaGraph_t g = nullptr;
     const long long counted = g_launches.load();
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    int r = launch_step(b, true, light);
-    if (!r) r = launch_step(b, true, light);
+    int r = launch_step(b, true, pass);
+    if (!r) r = launch_step(b, true, pass);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     g_launches = counted;  // capture recorded the launches without running them
     if (r) {
@@ -1834,7 +1841,7 @@ static int run_begin(impz_bunch_t b, const impz_elem_t* elems, int nelem) {
   b->run_wake = L.has_wake;
   if (b->run_wake && !b->wk_mem && (r = wake_alloc(b, 0))) return r;
   const int K = L.nsteps;
-  b->run_light = table_is_light(L.steps);
+  b->run_pass = table_pass(L.steps);
   if ((r = ensure_tables(b, K + 2, K + 1))) return r;
   if ((r = upload_lz_data(b, L.lz_data))) return r;
   if (b->sp_rec)  // every pass adds its blocks' counts to its record row
@@ -1847,7 +1854,7 @@ static int run_begin(impz_bunch_t b, const impz_elem_t* elems, int nelem) {
   CK(cudaMemcpyAsync(&b->st->step, &b->h_step0, sizeof(int), cudaMemcpyHostToDevice,
                      b->stream));
   AdvanceArgs a = advance_args(b, b->dsteps, -1, 0, 1, 1, b->mom_out, 0);
-  CK(launch_adv(b, a, step_is_light(L.steps[0])));
+  CK(launch_adv(b, a, step_pass(L.steps[0])));
   b->run_next = 1;
   return IMPZ_OK;
 }
@@ -1861,15 +1868,16 @@ static int run_advance(impz_bunch_t b, int budget) {
   int done = 0;
   while (b->run_next <= K && (done == 0 || done < budget)) {
     const int s = b->run_next;
-    const bool sc = L.steps[s].sc != 0, light = step_is_light(L.steps[s]);
+    const bool sc = L.steps[s].sc != 0;
+    const PassKind pass = step_pass(L.steps[s]);
     int r;
     if (!b->prof_on && sc && s + 1 <= K && L.steps[s + 1].sc &&
-        step_is_light(L.steps[s + 1]) == light) {
-      r = graph_pair(b, light);
+        step_pass(L.steps[s + 1]) == pass) {
+      r = graph_pair(b, pass);
       b->run_next += 2;
       done += 2;
     } else {
-      r = launch_step(b, sc, light);
+      r = launch_step(b, sc, pass);
       b->run_next += 1;
       done += 1;
     }
@@ -1944,9 +1952,10 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
   const impz_bunch_t b0 = bs[0];
   cudaStream_t s = b0->stream, s2 = b0->stream2;
   const bool f32 = b0->f32();
-  bool light = true, species = false;  // species: a member carries the species column
+  PassKind pass = PASS_LIGHT;
+  bool species = false;  // a member carries the species column
   for (int i = 0; i < nb; i++) {
-    light = light && bs[i]->run_light;
+    pass = wider(pass, bs[i]->run_pass);
     species = species || bs[i]->spc[0] != nullptr;
   }
   // the prologues ran on the bunches' own streams
@@ -2076,8 +2085,8 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
       if ((e = cudaStreamWaitEvent(s, b0->ev_scan, 0)) != cudaSuccess) return e;
     }
     const AdvanceArgs* a = d_adv + (size_t)(sc ? p : 2 + p) * nb;
-    e = f32 ? fast::launch_advance_packed(a, d_ao, nb, n_adv, true, light, species, s)
-            : exact::launch_advance_packed(a, d_ao, nb, n_adv, false, light, species, s);
+    e = f32 ? fast::launch_advance_packed(a, d_ao, nb, n_adv, pass, species, s)
+            : exact::launch_advance_packed(a, d_ao, nb, n_adv, pass, species, s);
     g_launches += 1;
     return e;
   };
@@ -2142,7 +2151,7 @@ static size_t packed_scratch_bytes(int nb) {
          3 * round_up((size_t)(nb + 1) * sizeof(int), kAlign);
 }
 
-static int packed_step(impz_bunch_t* bs, int nb, char* dscratch, bool f32, bool light) {
+static int packed_step(impz_bunch_t* bs, int nb, char* dscratch, bool f32, PassKind pass) {
   const impz_bunch_t b0 = bs[0];  // its streams and events carry the packed launches
   cudaStream_t s = b0->stream, s2 = b0->stream2;
   cudaEvent_t evf = b0->ev_fork, evj = b0->ev_join;
@@ -2250,12 +2259,10 @@ static int packed_step(impz_bunch_t* bs, int nb, char* dscratch, bool f32, bool 
     g_launches += 2 + 9 * (int)groups.size();
     CK(cudaStreamWaitEvent(s, b0->ev_scan, 0));
   }
-  e = f32 ? fast::launch_advance_packed((const AdvanceArgs*)(dscratch + o_adv),
-                                        (const int*)(dscratch + o_ao), nm, adv_offs[nm], true,
-                                        light, species, s)
-          : exact::launch_advance_packed((const AdvanceArgs*)(dscratch + o_adv),
-                                         (const int*)(dscratch + o_ao), nm, adv_offs[nm], false,
-                                         light, species, s);
+  const AdvanceArgs* d_adv = (const AdvanceArgs*)(dscratch + o_adv);
+  const int* d_ao = (const int*)(dscratch + o_ao);
+  e = f32 ? fast::launch_advance_packed(d_adv, d_ao, nm, adv_offs[nm], pass, species, s)
+          : exact::launch_advance_packed(d_adv, d_ao, nm, adv_offs[nm], pass, species, s);
   if (e != cudaSuccess) return cuda_fail(e, "packed step: particle pass");
   g_launches += 1;
   for (impz_bunch_t b : mem_b) {
@@ -2269,7 +2276,7 @@ int impz_run_advance_packed(impz_bunch_t* bunches, int nb, int steps, int* remai
   if (!bunches || nb < 1 || steps < 1) return IMPZ_ERR_ARG;
   const impz_bunch_t b0 = bunches[0];
   if (!b0) return IMPZ_ERR_ARG;
-  bool light = true;
+  PassKind pass = PASS_LIGHT;
   std::vector<impz_bunch_t> pk;  // the packable ones; bunches with wakes step on their own
   for (int i = 0; i < nb; i++) {
     const impz_bunch_t b = bunches[i];
@@ -2284,7 +2291,7 @@ int impz_run_advance_packed(impz_bunch_t* bunches, int nb, int steps, int* remai
       if (r) return r;
     } else {
       pk.push_back(b);
-      light = light && b->run_light;
+      pass = wider(pass, b->run_pass);
     }
   }
   if (pk.empty()) {
@@ -2305,7 +2312,7 @@ int impz_run_advance_packed(impz_bunch_t* bunches, int nb, int steps, int* remai
   CK(cudaMallocAsync((void**)&dscratch, packed_scratch_bytes(np), s));
   int r = IMPZ_OK;
   for (int k = 0; k < steps && !r; k++)
-    r = packed_step(pk.data(), np, dscratch, b0->f32(), light);
+    r = packed_step(pk.data(), np, dscratch, b0->f32(), pass);
   cudaFreeAsync(dscratch, s);
   CK(cudaEventRecord(pk[0]->ev_dep, s));
   for (int i = 1; i < np; i++) CK(cudaStreamWaitEvent(pk[i]->stream, pk[0]->ev_dep, 0));
@@ -2473,7 +2480,7 @@ int impz_set_integrator(impz_bunch_t b, int flagmap) {
 
 static void drop_graphs(impz_bunch_t b) {
   cudaStreamSynchronize(b->stream);
-  for (int p = 0; p < 4; p++)
+  for (int p = 0; p < impz_bunch_s::kGraphs; p++)
     if (b->gexec[p]) {
       cudaGraphExecDestroy(b->gexec[p]);
       b->gexec[p] = nullptr;

@@ -90,6 +90,17 @@ enum LzKind {
   LZ_EMFLD = 10
 };
 
+// The instantiations of the particle pass.  Registers bound it (two particles
+// per thread at 128), so a step runs the smallest one its maps allow: the
+// Lorentz kick and the ideal RF gap alone take the full pass's stack frame from
+// 24 to 176 bytes a thread, and a pass of 2e7 electrons through sector bends
+// from 1239 to 1336 us.
+enum PassKind : int {
+  PASS_FULL = 0,   // every map, and the Lorentz kick
+  PASS_LIGHT = 1,  // MAP_DRIFT and MAP_XM2
+  PASS_MAPS = 2,   // every map but MAP_IDEALRF, without the Lorentz kick
+};
+
 struct MapProgram {
   int nops;
   int pad;

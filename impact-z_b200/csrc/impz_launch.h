@@ -48,16 +48,16 @@ inline cudaError_t launch_pdl(void (*kernel)(KP...), dim3 grid, dim3 block, size
 
 #define IMPZ_DECLARE_PARTICLE_LAUNCHERS(NS)                                              \
   namespace NS {                                                                         \
-  cudaError_t launch_advance(const AdvanceArgs& a, bool f32, bool light, int grid,       \
+  cudaError_t launch_advance(const AdvanceArgs& a, PassKind pass, int grid,              \
                              cudaStream_t s);                                            \
   cudaError_t launch_deposit(const DepositArgs& a, int grid, cudaStream_t s);            \
   cudaError_t launch_wake(const WakeArgs& a, int grid, cudaStream_t s);                  \
   cudaError_t prepare_wake();                                                            \
   cudaError_t launch_scan(int* counts, int* cursor, int* bsum, long long total,          \
                           DevState* st, cudaStream_t s);                                 \
-  int max_blocks_advance(bool f32);                                                      \
+  int max_blocks_advance();                                                              \
   cudaError_t launch_advance_packed(const AdvanceArgs* args, const int* offs, int nmem,  \
-                                    int blocks, bool f32, bool light, bool species,      \
+                                    int blocks, PassKind pass, bool species,             \
                                     cudaStream_t s);                                     \
   cudaError_t launch_deposit_packed(const DepositArgs* args, const int* offs, int nmem,  \
                                     int blocks, bool species, cudaStream_t s);            \

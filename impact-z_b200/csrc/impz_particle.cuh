@@ -394,14 +394,12 @@ __device__ __forceinline__ void map_sector(Particle& p, const volatile double* c
 // pointers inside the particle loop: the coefficients are re-read (a
 // broadcast shared load) per particle instead of being hoisted into
 // registers for every map kind the switch could take.
-// LIGHT programs hold only drifts and block-diagonal linear maps (the
-// drift/quadrupole lattices); the host picks that instantiation when every
-// step of a run qualifies, which keeps the other map kinds' code and
-// registers out of the particle pass.
+// The host picks the instantiation (PassKind) from a step's programs, which
+// keeps the code and registers of maps that do not occur out of the pass.
 // qmi: the particles' Pts1(7), read by the K-map and the bend maps.
 // Every op is applied to the thread's U particles in turn, so that a
 // coefficient's load serves them all and their arithmetic interleaves.
-template <bool LIGHT, int U>
+template <PassKind PASS, int U>
 __device__ __forceinline__ void apply_program(Particle (&p)[U], const volatile MapProgram& prog,
                                               const double (&qmi)[U]) {
   const int nops = prog.nops;
@@ -410,7 +408,7 @@ __device__ __forceinline__ void apply_program(Particle (&p)[U], const volatile M
   for (int o = 0; o < nops; o++) {
     const volatile MapOp& op = prog.ops[o];
     const int kind = op.kind;
-    if (LIGHT) {
+    if (PASS == PASS_LIGHT) {
       if (kind == MAP_DRIFT) { IMPZ_EACH(map_drift(p[u], op.c)) }
       else if (kind == MAP_XM2) { IMPZ_EACH(map_xm2(p[u], op.c)) }
       continue;
@@ -419,7 +417,9 @@ __device__ __forceinline__ void apply_program(Particle (&p)[U], const volatile M
       case MAP_DRIFT: IMPZ_EACH(map_drift(p[u], op.c)) break;
       case MAP_XM6: IMPZ_EACH(map_xm6(p[u], op.c, op.flags, op.iparam)) break;
       case MAP_KQUAD: IMPZ_EACH(map_kquad(p[u], op.c, qmi[u])) break;
-      case MAP_IDEALRF: IMPZ_EACH(map_idealrf(p[u], op.c, op.flags, op.iparam)) break;
+      case MAP_IDEALRF:
+        if (PASS == PASS_FULL) { IMPZ_EACH(map_idealrf(p[u], op.c, op.flags, op.iparam)) }
+        break;
       case MAP_FPOL: IMPZ_EACH(map_pole<false>(p[u], op.c, qmi[u])) break;
       case MAP_BPOL: IMPZ_EACH(map_pole<true>(p[u], op.c, qmi[u])) break;
       case MAP_SECTOR: IMPZ_EACH(map_sector(p[u], op.c, qmi[u])) break;
@@ -1063,7 +1063,7 @@ __device__ __forceinline__ void lorentz_kick(Particle& p, double exn, double eyn
 // that owns the block in a launch over many.
 // SP: the instantiation for multi-species bunches (the species column, each
 // particle's q/m and the per-species counts); without it that code is absent.
-template <int BLOCK, bool F32, int U, bool LIGHT, bool SP>
+template <int BLOCK, bool F32, int U, PassKind PASS, bool SP>
 __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx, const int vgx) {
   __shared__ double red[BLOCK / 32][IMPZ_RAW_LEN];
   __shared__ double redr[BLOCK / 32][8];
@@ -1210,7 +1210,7 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
         p[u].y = yg * xk;
         p[u].ph = zg * xk / (-(gam * betai));
 #endif
-        if (!LIGHT && sp->lorentz) {
+        if (PASS == PASS_FULL && sp->lorentz) {
           // scatter2_BeamBunch (BeamBunch.f90:2766-3065): the same way back
           // to the z frame, then the implicit Lorentz update
           // scatter2wake: the wake's planes kx, kx+1 weighted by the
@@ -1229,7 +1229,7 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
           p[u].pt = p[u].pt - tt * ezn;
         }
       }
-    } else if (!LIGHT && post && sp->lorentz) {
+    } else if (PASS == PASS_FULL && post && sp->lorentz) {
       // a Lorentz-integrator step without space charge: scatter20's kick by
       // the element's field alone, on the stored coordinates
       // (BeamBunch.f90:3075-3531)
@@ -1237,7 +1237,7 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
       for (int u = 0; u < U; u++)
         lorentz_kick(p[u], 0.0, 0.0, 0.0, gam, sp, a.k, 0.0, 0.0, 0.0, a.lz_data, qmi[u]);
     }
-    if (post) apply_program<LIGHT, U>(p, progs[0], qmi);
+    if (post) apply_program<PASS, U>(p, progs[0], qmi);
     if (mom) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
@@ -1247,7 +1247,7 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
       }
       warp_moments<U>(mtile_dyn + wid * 32 * IMPZ_MSUMS, c, lane, macc0, macc1, mmax);
     }
-    if (pre) apply_program<LIGHT, U>(p, progs[1], qmi);
+    if (pre) apply_program<PASS, U>(p, progs[1], qmi);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       if (keep[u] && !finite6(p[u])) err |= DERR_NONFINITE;
@@ -1451,9 +1451,9 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
   }
 }
 
-template <int BLOCK, bool F32, int U, bool LIGHT, bool SP>
+template <int BLOCK, bool F32, int U, PassKind PASS, bool SP>
 __global__ void __launch_bounds__(BLOCK, IMPZ_ADV_MINB) k_advance(AdvanceArgs a) {
-  advance_pass<BLOCK, F32, U, LIGHT, SP>(a, blockIdx.x, gridDim.x);
+  advance_pass<BLOCK, F32, U, PASS, SP>(a, blockIdx.x, gridDim.x);
 }
 
 // The member of a packed launch that owns block `blk`: blocks
@@ -1478,7 +1478,7 @@ __device__ __forceinline__ void copy_args(void* dst, const void* src, int bytes)
 
 // Every member's pass in one launch: a packed work list of (bunch, block)
 // items, each bunch keeping its own block count and last-block reduction.
-template <int BLOCK, bool F32, int U, bool LIGHT, bool SP>
+template <int BLOCK, bool F32, int U, PassKind PASS, bool SP>
 __global__ void __launch_bounds__(BLOCK, IMPZ_ADV_MINB)
     k_advance_packed(const AdvanceArgs* __restrict__ args, const int* __restrict__ offs,
                      int nmem) {
@@ -1487,7 +1487,7 @@ __global__ void __launch_bounds__(BLOCK, IMPZ_ADV_MINB)
   const int m = packed_member(offs, nmem, blockIdx.x);
   copy_args(&sa, args + m, (int)sizeof(AdvanceArgs));
   __syncthreads();
-  advance_pass<BLOCK, F32, U, LIGHT, SP>(sa, blockIdx.x - __ldg(offs + m),
+  advance_pass<BLOCK, F32, U, PASS, SP>(sa, blockIdx.x - __ldg(offs + m),
                                      __ldg(offs + m + 1) - __ldg(offs + m));
 }
 

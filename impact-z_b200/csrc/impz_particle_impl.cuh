@@ -10,57 +10,62 @@ static const size_t kDepSmem = (size_t)3 * IMPZ_DEP_TILE * sizeof(unsigned int);
 
 static const size_t kAdvSmem = (size_t)(IMPZ_ADV_BLOCK / 32) * 32 * 37 * sizeof(double);
 
-template <bool F32, bool LIGHT, bool SP>
+// the form this namespace is built for gathers an FP32 field or an FP64 one
+constexpr bool kF32 = IMPZ_FASTMATH != 0;
+
+template <PassKind PASS, bool SP>
 static cudaError_t adv_attr() {
   static cudaError_t once = cudaFuncSetAttribute(
-      k_advance<IMPZ_ADV_BLOCK, F32, IMPZ_ADV_U, LIGHT, SP>,
+      k_advance<IMPZ_ADV_BLOCK, kF32, IMPZ_ADV_U, PASS, SP>,
       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdvSmem);
   return once;
 }
 
-template <bool F32, bool LIGHT, bool SP>
+template <PassKind PASS, bool SP>
 static cudaError_t launch_adv_t(const AdvanceArgs& a, int grid, cudaStream_t s) {
-  cudaError_t e = adv_attr<F32, LIGHT, SP>();
+  cudaError_t e = adv_attr<PASS, SP>();
   if (e != cudaSuccess) return e;
-  return launch_pdl(k_advance<IMPZ_ADV_BLOCK, F32, IMPZ_ADV_U, LIGHT, SP>, dim3(grid),
+  return launch_pdl(k_advance<IMPZ_ADV_BLOCK, kF32, IMPZ_ADV_U, PASS, SP>, dim3(grid),
                     dim3(IMPZ_ADV_BLOCK), kAdvSmem, s, a);
 }
 
-template <bool F32, bool LIGHT>
+template <PassKind PASS>
 static cudaError_t launch_adv_sp(const AdvanceArgs& a, int grid, cudaStream_t s) {
-  return a.sp_in ? launch_adv_t<F32, LIGHT, true>(a, grid, s)
-                 : launch_adv_t<F32, LIGHT, false>(a, grid, s);
+  return a.sp_in ? launch_adv_t<PASS, true>(a, grid, s) : launch_adv_t<PASS, false>(a, grid, s);
 }
 
-cudaError_t launch_advance(const AdvanceArgs& a, bool f32, bool light, int grid, cudaStream_t s) {
-  if (f32) return light ? launch_adv_sp<true, true>(a, grid, s) : launch_adv_sp<true, false>(a, grid, s);
-  return light ? launch_adv_sp<false, true>(a, grid, s) : launch_adv_sp<false, false>(a, grid, s);
+cudaError_t launch_advance(const AdvanceArgs& a, PassKind pass, int grid, cudaStream_t s) {
+  switch (pass) {
+    case PASS_LIGHT: return launch_adv_sp<PASS_LIGHT>(a, grid, s);
+    case PASS_MAPS: return launch_adv_sp<PASS_MAPS>(a, grid, s);
+    default: return launch_adv_sp<PASS_FULL>(a, grid, s);
+  }
 }
 
-template <bool F32, bool LIGHT, bool SP>
+template <PassKind PASS, bool SP>
 static cudaError_t launch_adv_packed_t(const AdvanceArgs* args, const int* offs, int nmem,
                                        int blocks, cudaStream_t s) {
-  auto kern = k_advance_packed<IMPZ_ADV_BLOCK, F32, IMPZ_ADV_U, LIGHT, SP>;
+  auto kern = k_advance_packed<IMPZ_ADV_BLOCK, kF32, IMPZ_ADV_U, PASS, SP>;
   static cudaError_t once =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdvSmem);
   if (once != cudaSuccess) return once;
   return launch_pdl(kern, dim3(blocks), dim3(IMPZ_ADV_BLOCK), kAdvSmem, s, args, offs, nmem);
 }
 
-template <bool F32, bool LIGHT>
+template <PassKind PASS>
 static cudaError_t launch_adv_packed_sp(const AdvanceArgs* args, const int* offs, int nmem,
                                         int blocks, bool species, cudaStream_t s) {
-  return species ? launch_adv_packed_t<F32, LIGHT, true>(args, offs, nmem, blocks, s)
-                 : launch_adv_packed_t<F32, LIGHT, false>(args, offs, nmem, blocks, s);
+  return species ? launch_adv_packed_t<PASS, true>(args, offs, nmem, blocks, s)
+                 : launch_adv_packed_t<PASS, false>(args, offs, nmem, blocks, s);
 }
 
 cudaError_t launch_advance_packed(const AdvanceArgs* args, const int* offs, int nmem, int blocks,
-                                  bool f32, bool light, bool species, cudaStream_t s) {
-  if (f32)
-    return light ? launch_adv_packed_sp<true, true>(args, offs, nmem, blocks, species, s)
-                 : launch_adv_packed_sp<true, false>(args, offs, nmem, blocks, species, s);
-  return light ? launch_adv_packed_sp<false, true>(args, offs, nmem, blocks, species, s)
-               : launch_adv_packed_sp<false, false>(args, offs, nmem, blocks, species, s);
+                                  PassKind pass, bool species, cudaStream_t s) {
+  switch (pass) {
+    case PASS_LIGHT: return launch_adv_packed_sp<PASS_LIGHT>(args, offs, nmem, blocks, species, s);
+    case PASS_MAPS: return launch_adv_packed_sp<PASS_MAPS>(args, offs, nmem, blocks, species, s);
+    default: return launch_adv_packed_sp<PASS_FULL>(args, offs, nmem, blocks, species, s);
+  }
 }
 
 template <bool SP>
@@ -140,20 +145,14 @@ cudaError_t launch_species_count(const DepositArgs& a, int test_loss, int nspeci
   return cudaGetLastError();
 }
 
-int max_blocks_advance(bool f32) {
+int max_blocks_advance() {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // the full multi-species instantiation bounds the others (at most its registers)
-  if (f32) {
-    adv_attr<true, false, true>();
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per, k_advance<IMPZ_ADV_BLOCK, true, IMPZ_ADV_U, false, true>, IMPZ_ADV_BLOCK, kAdvSmem);
-  } else {
-    adv_attr<false, false, true>();
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per, k_advance<IMPZ_ADV_BLOCK, false, IMPZ_ADV_U, false, true>, IMPZ_ADV_BLOCK, kAdvSmem);
-  }
+  adv_attr<PASS_FULL, true>();
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per, k_advance<IMPZ_ADV_BLOCK, kF32, IMPZ_ADV_U, PASS_FULL, true>, IMPZ_ADV_BLOCK, kAdvSmem);
   return sms * (per > 0 ? per : 1);
 }
 
