@@ -25,4 +25,11 @@ __device__ __forceinline__ void griddep_launch() {
 #endif
 }
 
+// Brings the 128-byte line at p into L2, without waiting and without a register.
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+#if defined(__CUDA_ARCH__)
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+#endif
+}
+
 }  // namespace impz
