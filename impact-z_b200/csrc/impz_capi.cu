@@ -2467,9 +2467,9 @@ int impz_run_reference(impz_bunch_t b, double* refrec, int maxrec, int* nrec) {
 
 // ---- autotuner ------------------------------------------------------------
 // Times real runs of the bunch (nsteps space-charge steps of a short drift)
-// under candidate launch shapes: deposit and push blocks, and z lines per
-// block of the convolution; one parameter at a time, keeping the best.
-// The bunch is restored before each trial and at the end.
+// under candidate launch shapes: deposit and push blocks, one parameter at a
+// time, keeping the best.  The bunch is restored before each trial and at the
+// end.
 int impz_step_params_size(void) { return (int)sizeof(StepParams); }
 
 int impz_set_integrator(impz_bunch_t b, int flagmap) {

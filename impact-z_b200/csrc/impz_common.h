@@ -251,7 +251,7 @@ struct WakeArgs {
 
 // One bunch of a group of bunches with the same grid size and form, for the
 // field solve launched once for the whole group (the *_group kernels):
-// blockIdx.y or blockIdx.z selects the member.
+// blockIdx.y selects the member.
 struct PoissonMember {
   unsigned long long* rho;  // int64 charge (read by the forward pass, cleared by the field)
   double qscale;            // grid value of one fixed-point quantum

@@ -355,7 +355,7 @@
           end function
 
           ! launch shapes for this bunch: out = deposit blocks, push blocks,
-          ! z lines per block, ms per step
+          ! 0, ms per step
           integer(c_int) function impz_autotune(bunch, nsteps, out) &
               bind(C, name="impz_autotune")
             import :: c_int, c_double, c_ptr
