@@ -2124,6 +2124,7 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
       st += 1;
     }
   }
+  if (rc) cudaStreamSynchronize(s2);  // a failed step's Green build or scan reads dmem
   const cudaError_t es = cudaStreamSynchronize(s);
   for (int k = 0; k < 2; k++)
     if (gx[k]) cudaGraphExecDestroy(gx[k]);
@@ -2313,9 +2314,17 @@ int impz_run_advance_packed(impz_bunch_t* bunches, int nb, int steps, int* remai
   int r = IMPZ_OK;
   for (int k = 0; k < steps && !r; k++)
     r = packed_step(pk.data(), np, dscratch, b0->f32(), pass);
+  // a step that failed between two launches leaves its Green build or its scan
+  // on the second stream, which read dscratch and the members' grids
+  if (r) cudaStreamSynchronize(pk[0]->stream2);
   cudaFreeAsync(dscratch, s);
-  CK(cudaEventRecord(pk[0]->ev_dep, s));
-  for (int i = 1; i < np; i++) CK(cudaStreamWaitEvent(pk[i]->stream, pk[0]->ev_dep, 0));
+  cudaError_t e = cudaEventRecord(pk[0]->ev_dep, s);
+  for (int i = 1; i < np && e == cudaSuccess; i++)
+    e = cudaStreamWaitEvent(pk[i]->stream, pk[0]->ev_dep, 0);
+  if (e != cudaSuccess) {  // the members' own streams could not be put behind s
+    cudaStreamSynchronize(s);
+    if (!r) r = cuda_fail(e, "packed advance: joining the members' streams");
+  }
   for (int i = 0; i < nb; i++) {
     impz_bunch_t b = bunches[i];
     if (remaining) remaining[i] = std::max(0, b->lat.nsteps + 1 - b->run_next);
