@@ -526,6 +526,16 @@ struct impz_bunch_s {
 
 namespace {
 
+// Kernels per launch wrapper, for the launch count: the Green build (corners,
+// xy, z), the field solve of one bunch or of a group (with the transform
+// forward, along z and back, and the field), and a space-charge step (with the
+// deposit, the count scan and the push).
+constexpr int kGreenKernels = 3, kSolveKernels = kGreenKernels + 3 + 1, kWakeKernels = 2;
+constexpr int packed_kernels(int groups) { return kSolveKernels * groups + 3; }
+int step_kernels(impz_bunch_t b) {
+  return packed_kernels(1) + (b->run_wake ? kWakeKernels : 0);
+}
+
 // CUDA events around one kernel group (only when profiling is on)
 struct ProfScope {
   impz_bunch_t b;
@@ -703,7 +713,7 @@ cudaError_t launch_deposit(impz_bunch_t b, const DepositArgs& d) {
 }
 
 int solve_green(impz_bunch_t b, cudaStream_t s) {
-  ProfScope ps(b, IMPZ_PROF_GREEN, 5, s);
+  ProfScope ps(b, IMPZ_PROF_GREEN, kGreenKernels, s);
   PoissonBuffers pb = poisson_of(b);
   if (b->f32()) { CK(launch_green<float>(pb, s)); }
   else { CK(launch_green<double>(pb, s)); }
@@ -761,7 +771,7 @@ int field_step(impz_bunch_t b, const StepParams* table, int fixed) {
   }
   if (!serial) CK(cudaEventRecord(b->ev_scan, b->stream2));
   if (b->run_wake) {
-    ProfScope ps(b, IMPZ_PROF_WAKE, 2);
+    ProfScope ps(b, IMPZ_PROF_WAKE, kWakeKernels);
     CK(exact::launch_wake(wake_args(b, table, fixed), b->grid_wake, b->stream));
   }
   PoissonBuffers pb = poisson_of(b);
@@ -1011,6 +1021,7 @@ void free_bunch(impz_bunch_t b) {
 // =====================================================================
 namespace impz {
 int report_cuda_error(cudaError_t e, const char* where) { return cuda_fail(e, where); }
+void count_launches(int kernels) { g_launches += kernels; }
 }  // namespace impz
 
 extern "C" {
@@ -1798,17 +1809,16 @@ static int graph_pair(impz_bunch_t b, PassKind pass) {
   }
   if (!b->gexec[k]) {
     cudaGraph_t g = nullptr;
-    const long long counted = g_launches.load();
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     int r = launch_step(b, true, pass);
     if (!r) r = launch_step(b, true, pass);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-    g_launches = counted;  // capture recorded the launches without running them
     if (r) {
       if (g) cudaGraphDestroy(g);
       return r;
     }
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
+    g_launches -= 2 * step_kernels(b);  // counted as they were captured, without running
     e = cudaGraphInstantiate(&b->gexec[k], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
@@ -1818,7 +1828,7 @@ static int graph_pair(impz_bunch_t b, PassKind pass) {
     b->g_lzd[k] = b->lzd;
     b->parity = p;  // capture did not execute anything
   }
-  g_launches += 2 * (12 + (b->run_wake ? 2 : 0));
+  g_launches += 2 * step_kernels(b);
   CK(cudaGraphLaunch(b->gexec[k], b->stream));
   return IMPZ_OK;
 }
@@ -2041,7 +2051,7 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
   const int* d_do = (const int*)(dmem + o_do);
   const int* d_so = (const int*)(dmem + o_so);
   const int n_adv = adv_offs[nb], n_dep = dep_offs[nb], n_scan = scan_offs[nb];
-  const int nlaunch_sc = 3 + 9 * (int)groups.size();
+  const int nlaunch_sc = packed_kernels((int)groups.size());
 
   // one step from parity p: the field solve and the kick (sc), or the pass alone
   auto step = [&](int p, bool sc) -> cudaError_t {
@@ -2100,7 +2110,6 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
     if (sc && st + 1 <= K && b0->lat.steps[st + 1].sc) {
       if (!gx[p]) {
         cudaGraph_t g = nullptr;
-        const long long counted = g_launches.load();
         cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
           cudaError_t e1 = step(p, true);
@@ -2108,8 +2117,10 @@ static int run_batch_packed(impz_bunch_t* bs, int nb) {
           e = cudaStreamEndCapture(s, &g);
           if (e2 != cudaSuccess) e = e2;
         }
-        g_launches = counted;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&gx[p], g, 0);
+        if (e == cudaSuccess) {
+          g_launches -= 2 * nlaunch_sc;  // counted as they were captured, without running
+          e = cudaGraphInstantiate(&gx[p], g, 0);
+        }
         if (g) cudaGraphDestroy(g);
         if (e != cudaSuccess) { rc = cuda_fail(e, "packed batch graph"); break; }
       }
@@ -2257,7 +2268,7 @@ static int packed_step(impz_bunch_t* bs, int nb, char* dscratch, bool f32, PassK
                 : launch_efield_group<double>(g.nx, g.ny, g.nz, d_mem + g.first, g.count, s);
       if (e != cudaSuccess) return cuda_fail(e, "packed step: field solve");
     }
-    g_launches += 2 + 9 * (int)groups.size();
+    g_launches += packed_kernels((int)groups.size()) - 1;  // all but the pass
     CK(cudaStreamWaitEvent(s, b0->ev_scan, 0));
   }
   const AdvanceArgs* d_adv = (const AdvanceArgs*)(dscratch + o_adv);

@@ -146,5 +146,7 @@ IMPZ_DECLARE_POISSON(double)
 // Records a CUDA failure for impz_last_cuda_error and returns IMPZ_ERR_CUDA
 // (for translation units other than the C-ABI core).
 int report_cuda_error(cudaError_t e, const char* where);
+// Adds to impz_kernel_launches (for the same units).
+void count_launches(int kernels);
 
 }  // namespace impz

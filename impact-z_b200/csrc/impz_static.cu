@@ -183,5 +183,6 @@ extern "C" int impz_deposit_static(const double* x, const double* px, const doub
     e = launch_pdl(k_static_finish, dim3(gclear), dim3(256), 0, s, (const unsigned long long*)acc,
                    G, a.scale, chgdens);
   if (e != cudaSuccess) return report_cuda_error(e, "impz_deposit_static: launch");
+  count_launches(n > 0 ? 3 : 2);
   return IMPZ_OK;
 }

@@ -5,6 +5,9 @@ A packed advance whose k-th enqueued operation fails, for every k, returns the
 error and frees its argument memory only after everything it had enqueued, on
 both streams.
 
+impz_kernel_launches counts the kernels that ran: in every call that launches
+any, by direct launches and by graph replay alike.
+
 The process (a child: the library is loaded a second time) is given the linked
 library's path."""
 import ctypes
@@ -50,6 +53,11 @@ def run_child(fake_lib, what):
 
 def test_a_failed_packed_advance_frees_its_arguments_after_all_its_work(fake_lib):
     run_child(fake_lib, "packed_failures")
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
+def test_the_launch_count_is_the_number_of_kernels(fake_lib, form):
+    run_child(fake_lib, "launch_counts_" + form)
 
 
 # ---- in the child ---------------------------------------------------------
@@ -100,5 +108,65 @@ def packed_failures():
     assert not bad, "%d of %d: %s" % (len(bad), total, bad)
 
 
+def launch_counts(form):
+    impz, L, beams = setup()
+    from test_wake import synthetic_table
+
+    def counted(what, f, want=None):
+        c0, k0 = impz.kernel_launches(), L.fake_kernels()
+        f()
+        c, k = impz.kernel_launches() - c0, L.fake_kernels() - k0
+        assert c == k, (what, c, k)
+        assert want is None or c == want, (what, c, want)
+
+    drift = impz.elem(0, 0.1, 4, 1, [1.0])
+    for grid in ((8, 8, 16), (64, 16, 8)):
+        b = make(impz, beams, 700, grid, form)
+        counted("map", lambda: b.map_half(drift, 0.0, 0.0, 0.0125, 1, 0), 1)
+        counted("prepare", lambda: b.sc_prepare(1.0, 1.0))
+        counted("deposit", lambda: b.deposit(), 3)
+        counted("poisson", lambda: b.poisson())
+        counted("kick", lambda: b.kick(0.025, want_e=True))
+        counted("moments", lambda: b.moments())
+        counted("bunching", lambda: b.bunching(1e3))
+        # a prologue, then ten kernels a step: in pairs from a graph, and singly
+        counted("capture", lambda: b.run([drift]), 1 + 4 * 10)
+        counted("replay", lambda: b.run([drift]), 1 + 4 * 10)
+        counted("odd", lambda: b.run([impz.elem(0, 0.1, 3, 1, [1.0])]), 1 + 3 * 10)
+        b.wake(synthetic_table(), 1.0, True)
+        counted("wake", lambda: b.run([drift]), 1 + 4 * 12)
+        b.wake_off()
+        b.profile_enable(True)
+        counted("profile", lambda: b.run([drift]), 1 + 4 * 10)
+        b.profile_enable(False)
+        c = beams.fodo_1e5(n=700)
+        counted("upload", lambda: b.upload(c["pts"], c["current"], c["refptcl"]))
+        counted("download", lambda: b.download())
+        b.close()
+    # groups: the field solve once per grid size, the rest once
+    grids = [(8, 8, 16), (16, 8, 16), (8, 8, 16)]
+    for group, per in (((0, 2), 10), ((0, 1, 2), 17)):
+        bs = [make(impz, beams, 500, grids[k], form) for k in group]
+        lats = [[drift]] * len(bs)
+        for _ in range(2):
+            counted("batch", lambda: impz.run_batch(bs, lats), len(bs) + 4 * per)
+            counted("packed", lambda: impz.run_packed(bs, lats, 3), len(bs) + 4 * per)
+        for b in bs:
+            b.close()
+    # the deposit into the caller's memory (host memory here)
+    x = [np.zeros(64) for _ in range(6)]
+    box = np.array([-1.0, 1.0] * 3)
+    out = np.zeros(8 * 8 * 8)
+    for n, want in ((64, 3), (0, 2)):
+        counted("static", lambda: L.impz_deposit_static(
+            *[a.ctypes.data for a in x], n, 2.0, 1.0, 1.0, 4e8, 1.0,
+            box.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), 8, 8, 8, out.ctypes.data, None),
+            want)
+
+
 if __name__ == "__main__":
-    {"packed_failures": packed_failures}[sys.argv[1]]()
+    if sys.argv[1] == "packed_failures":
+        packed_failures()
+    else:
+        form = load_impz().FORM_FP64 if sys.argv[1].endswith("64") else load_impz().FORM_FP32CONV
+        launch_counts(form)
