@@ -16,7 +16,7 @@
 // Twiddles come from a table in the order the threads read them: stage with
 // Ns points done holds exp(-2 pi i e m / (Ns R)), e = 1..R-1 by m = 0..Ns-1,
 // from entry Ns - E on (the stages' sizes telescope, so a table has N - E
-// entries).  They are correctly rounded table values, never products.
+// entries).  They are rounded once from the exact angle, never products.
 #pragma once
 #include <cuda_runtime.h>
 

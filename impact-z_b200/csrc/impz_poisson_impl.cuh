@@ -203,6 +203,25 @@ cudaError_t efield(const PoissonDims& d, const Members& m, const double* wake,
                     wake_line);
 }
 
+// exp(-2 pi i k / 2^logn), logn >= 3: the angle is reduced to the first
+// octant as an integer, so that it is rounded once, in extended precision,
+// and the multiples of an eighth of a turn come out as they are.  An angle
+// up to a full turn in FP64 put the entries several units in the last place
+// off.
+void unit_root(int logn, long long k, long double& re, long double& im) {
+  const long long n = 1ll << logn, eighth = n >> 3;
+  k &= n - 1;
+  const long long octant = k / eighth, rest = k & (eighth - 1);
+  const bool odd = octant & 1;  // counted back from the octant's end
+  const long double a = 2.0L * 3.14159265358979323846264338327950288L *
+                        (long double)(odd ? eighth - rest : rest) / (long double)n;
+  const long double c = std::cos(a), s = std::sin(a);
+  const long double x[4] = {c, s, -s, -c}, y[4] = {s, c, c, s};  // cos and sin, octants 0..3
+  const int o = (int)octant & 3;
+  re = octant < 4 ? x[o] : -x[o];
+  im = octant < 4 ? -y[o] : y[o];
+}
+
 }  // namespace
 
 // Twiddles of a transform of 2^logn points in the order the stages of
@@ -219,9 +238,10 @@ int fft_twiddles<IMPZ_POISSON_T>(int logn, void* out) {
     const int ns = 1 << lns, r = 1 << lr;
     for (int e = 1; e < r; e++)
       for (int m = 0; m < ns; m++, n++) {
-        const double a = -2.0 * M_PI * (double)e * (double)m / (double)(ns * r);
-        t[n].x = (IMPZ_POISSON_T)std::cos(a);
-        t[n].y = (IMPZ_POISSON_T)std::sin(a);
+        long double x, y;
+        unit_root(lns + lr, (long long)e * m, x, y);
+        t[n].x = (IMPZ_POISSON_T)x;
+        t[n].y = (IMPZ_POISSON_T)y;
       }
     lns += lr;
   }
