@@ -20,8 +20,8 @@ pytestmark = pytest.mark.gpu
 impz = load_impz()
 from impz_b200 import beams  # noqa: E402
 
-SIZES = [(4, 4, 4), (8, 4, 8), (4, 8, 16), (16, 16, 16), (8, 32, 32), (64, 8, 64), (32, 64, 256),
-         (16, 8, 512), (64, 64, 1024), (4, 16, 2048), (8, 8, 4096)]
+SIZES = [(4, 4, 4), (8, 4, 8), (4, 8, 16), (16, 16, 16), (8, 32, 32), (64, 8, 64), (32, 16, 128),
+         (32, 64, 256), (16, 8, 512), (64, 64, 1024), (4, 16, 2048), (8, 8, 4096)]
 
 
 @pytest.mark.parametrize("form,tol", [(impz.FORM_FP64, 1e-12), (impz.FORM_FP32CONV, 1e-6)])
@@ -38,7 +38,8 @@ def test_potential_at_every_length(grid, form, tol):
 
 
 @pytest.mark.parametrize("form", [impz.FORM_FP64, impz.FORM_FP32CONV])
-@pytest.mark.parametrize("grid", [(4, 8, 16), (16, 16, 16), (8, 8, 4096), (64, 64, 32)])
+@pytest.mark.parametrize("grid", [(4, 8, 16), (16, 16, 16), (8, 8, 4096), (64, 64, 32), (16, 16, 128),
+                                  (16, 16, 256)])
 def test_group_equals_solo(grid, form):
     def make(k):
         cfg = beams.fodo_1e5(n=3000 + 1111 * k, seed=beams.SEED0 + 92 + k)

@@ -164,3 +164,34 @@ def test_static_deposit_empty_beam_and_side_stream():
     side = torch.cuda.Stream()
     got = static_deposit(cfg, rng, 1.0, stream=side.cuda_stream)
     np.testing.assert_array_equal(got, first)
+
+
+@pytest.mark.gpu
+def test_static_deposit_in_a_callers_graph():
+    """Captured on the caller's stream and replayed twice, with other particles
+    the second time: each replay equals the direct call, so the early launches
+    inside the call keep its order when they become graph edges."""
+    import torch
+    beams_ = [beams.fodo_1e5(n=20_000, seed=beams.SEED0 + 25 + k) for k in range(2)]
+    rng = np.ascontiguousarray(bunch_deposit(beams_[0], 1.0)[1])
+    want = [static_deposit(cfg, rng, 1.0) for cfg in beams_]
+    dev = [[torch.from_numpy(np.ascontiguousarray(cfg["pts"][:, c])).to("cuda") for c in range(6)]
+           for cfg in beams_]
+    cols = [c.clone() for c in dev[0]]
+    cfg = beams_[0]
+    nx, ny, nz = cfg["grid"]
+    out = torch.full((nx * ny * nz,), float("nan"), dtype=torch.float64, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        rc = impz.lib().impz_deposit_static(
+            *[c.data_ptr() for c in cols], 20_000, -cfg["refptcl"][5], 1.0, 1.0, cfg["freq"],
+            float(cfg["pts"][0, 7]), rng.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
+            nx, ny, nz, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == impz.OK, impz.error_string(rc)
+    for k in (0, 1, 0):
+        for c, src in zip(cols, dev[k]):
+            c.copy_(src)
+        graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy(), want[k])
