@@ -91,10 +91,13 @@ enum LzKind {
 };
 
 // The instantiations of the particle pass.  Registers bound it (two particles
-// per thread at 128), so a step runs the smallest one its maps allow: the
-// Lorentz kick and the ideal RF gap alone take the full pass's stack frame from
-// 24 to 176 bytes a thread, and a pass of 2e7 electrons through sector bends
-// from 1239 to 1336 us.
+// per thread at 128), so a step of a run on its own takes the smallest one its
+// maps allow.  Bytes of stack frame (spill stores/loads) a thread, one species,
+// by -Xptxas -v: light 0 (0/0) in the FP32 form and 32 (60/60) in the FP64 one,
+// maps 128 (188/204) and 192 (368/444), full 168 (304/344) and 208 (408/488).
+// Measured in the FP32 form, 2e7 electrons through sector bends: full 1336 us,
+// maps 1239.  A packed launch of several bunches takes one instantiation, the
+// widest any of its members' runs needs at any step.
 enum PassKind : int {
   PASS_FULL = 0,   // every map, and the Lorentz kick
   PASS_LIGHT = 1,  // MAP_DRIFT and MAP_XM2

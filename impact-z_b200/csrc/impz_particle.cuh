@@ -586,30 +586,6 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
 __device__ __forceinline__ void raise_to(double& m, double x) { m = x > m ? x : m; }
 __device__ __forceinline__ void lower_to(double& m, double x) { m = x < m ? x : m; }
 
-// the 37 sums of diagnostic1_Output (Output.f90:133-196), in tmplc order
-__device__ __forceinline__ void moment_accumulate(double* s, const Particle& p) {
-  const double x = p.x, px = p.px, y = p.y, py = p.py, z = p.ph, pz = p.pt;
-  s[0] += x;  s[1] += px; s[2] += y;  s[3] += py; s[4] += z;  s[5] += pz;
-  s[6] += x * x; s[7] += px * px; s[8] += y * y; s[9] += py * py;
-  s[10] += z * z; s[11] += pz * pz;
-  s[12] += x * px; s[13] += y * py; s[14] += z * pz;
-  s[15] += x * x * x; s[16] += x * x * x * x;
-  s[17] += px * px * px; s[18] += px * px * px * px;
-  s[19] += y * y * y; s[20] += y * y * y * y;
-  s[21] += py * py * py; s[22] += py * py * py * py;
-  s[23] += fabs(z * z * z); s[24] += z * z * z * z;
-  s[25] += pz * pz * pz; s[26] += pz * pz * pz * pz;
-  s[27] += x * px * px; s[28] += x * px * px * px; s[29] += x * x * px;
-  s[30] += x * x * px * px; s[31] += x * x * x * px;
-  s[32] += y * py * py; s[33] += y * py * py * py; s[34] += y * y * py;
-  s[35] += y * y * py * py; s[36] += y * y * y * py;
-  s[37] = fmax(s[37], fabs(x)); s[38] = fmax(s[38], fabs(px));
-  s[39] = fmax(s[39], fabs(y)); s[40] = fmax(s[40], fabs(py));
-  s[41] = fmax(s[41], fabs(z)); s[42] = fmax(s[42], fabs(pz));
-  s[43] = fmax(s[43], x * x + y * y);
-}
-
-
 template <bool F32>
 __device__ __forceinline__ void gather_e(const void* ef, const Cell& c, int nx, int ny,
                                          double& ex, double& ey, double& ez);
@@ -1124,7 +1100,9 @@ __device__ __forceinline__ void advance_pass(const AdvanceArgs& a, const int vbx
   // are clamped like any other's) is dropped where something is kept.  With
   // a particle's chain behind its own branch the pass of 4e6 particles took
   // 227 us (220 so), that of 2e7 electrons mostly in sector bends 1502
-  // (1349).  Reciprocals and square roots of our own without the library
+  // (1349), both in the FP32 form.  The FP64 form's light pass gains nothing
+  // by it: 60 bytes a thread spilled, 102 us before and 105 so at 1e6
+  // particles.  Reciprocals and square roots of our own without the library
   // functions' special-case branches were slower (238).
   for (long long i0 = (long long)vbx * BLOCK * U + threadIdx.x; i0 < nround; i0 += stride) {
     Particle p[U];
