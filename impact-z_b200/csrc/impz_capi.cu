@@ -394,8 +394,8 @@ Layout plan_layout(long long n, int nx, int ny, int nz, int form, int flags) {
   L.ghat = take(noct * esz);
   L.phi = take(G * esz);
   L.efield = take(4 * G * esz);
-  const int half[3] = {nx, ny, nz};  // a length-2m transform keeps up to 2m twiddles
-  for (int d = 0; d < 3; d++) L.tw[d] = take((size_t)half[d] * 2 * 2 * esz);
+  const int half[3] = {nx, ny, nz};  // 16 bytes a point of the doubled length (fft_twiddles)
+  for (int d = 0; d < 3; d++) L.tw[d] = take((size_t)half[d] * 2 * sizeof(double2));
   L.st = take(sizeof(DevState));
   L.dfine = take(2 * sizeof(StepParams));
   L.mom_fine = take(IMPZ_MOMREC * sizeof(double));
@@ -1147,11 +1147,10 @@ int impz_bunch_create(const double* pts, long long n, double current, double mas
   ALLOC(cudaMemsetAsync(b->counts, 0, (G + 1) * sizeof(int), b->stream));
   const int lens[3] = {2 * nx, 2 * ny, 2 * nz};
   for (int d = 0; d < 3; d++) {
-    std::vector<double2> t(lens[d]);
-    const int m = b->f32() ? fft_twiddles<float>(ilog2i(lens[d]), t.data())
-                           : fft_twiddles<double>(ilog2i(lens[d]), t.data());
-    ALLOC(cudaMemcpy(b->tw[d], t.data(), (size_t)m * (b->f32() ? sizeof(float2) : sizeof(double2)),
-                     cudaMemcpyHostToDevice));
+    std::vector<double2> t(lens[d], double2{0.0, 0.0});
+    if (b->f32()) fft_twiddles<float>(ilog2i(lens[d]), t.data());
+    else fft_twiddles<double>(ilog2i(lens[d]), t.data());
+    ALLOC(cudaMemcpy(b->tw[d], t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
   }
   b->grid_adv = (int)std::min<long long>((n + IMPZ_ADV_BLOCK - 1) / IMPZ_ADV_BLOCK,
                                          (long long)(b->f32() ? fast::max_blocks_advance()

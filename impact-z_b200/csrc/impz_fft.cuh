@@ -16,7 +16,22 @@
 // Twiddles come from a table in the order the threads read them: stage with
 // Ns points done holds exp(-2 pi i e m / (Ns R)), e = 1..R-1 by m = 0..Ns-1,
 // from entry Ns - E on (the stages' sizes telescope, so a table has N - E
-// entries).  They are rounded once from the exact angle, never products.
+// entries).  They are rounded once from the exact angle, never products.  An
+// FP32 table has what the rounding dropped from entry N on.
+//
+// Rounded constants are not harmless in FP32.  The butterflies use the same few
+// in every line (cos pi/8 is 3e-8 short), and the first stage's meet the same
+// stretches of a line each time: a gain that depends on the position.  The
+// entries of the low harmonics turn +k and -k by different angles: a shift.
+// Either gives a bunch a net force of its own field, the same in every bunch
+// and every step: 9e-9 of the rms force along x and 6e-9 along y at 64x64x128,
+// where radix-2 transforms had 4e-9 of random sign and their centroids came out
+// five to ten times as close.  So the butterflies' constants have a second term
+// (c_mulc), everywhere, and the twiddles too (FINE) in the transforms along x
+// and y: net means below 1e-9, rms 2e-9 and 3e-9, the potential's error 1.10e-7
+// -> 0.92e-7, the rms momenta over 20 steps of 4e6 particles 9.4e-8 -> 1.4e-8.
+// Along z the net force was no worse than before, and second terms of its
+// tables cost (64x64x512: 311 -> 335 us a step, 64x64x4096: 2.0 -> 4.1 ms).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -52,6 +67,29 @@ __device__ __forceinline__ C c_mulw(C a, C w) {
   }
   return r;
 }
+// a * (w + l), conjugated likewise: l is what the rounding of w dropped
+template <int SIGN, typename C>
+__device__ __forceinline__ C c_mulw2(C a, C w, C l) {
+  C r;
+  if (SIGN < 0) {
+    r.x = fft_fma(a.x, w.x, fft_fma(-a.y, w.y, fft_fma(a.x, l.x, -(a.y * l.y))));
+    r.y = fft_fma(a.x, w.y, fft_fma(a.y, w.x, fft_fma(a.x, l.y, a.y * l.x)));
+  } else {
+    r.x = fft_fma(a.x, w.x, fft_fma(a.y, w.y, fft_fma(a.x, l.x, a.y * l.y)));
+    r.y = fft_fma(a.y, w.x, fft_fma(-a.x, w.y, fft_fma(a.y, l.x, -(a.x * l.y))));
+  }
+  return r;
+}
+// a * (c + i s), a constant of the butterflies, with its second term in FP32
+template <int SIGN, typename T, typename C>
+__device__ __forceinline__ C c_mulc(C a, double c, double s) {
+  C w, l;
+  w.x = (T)c;
+  w.y = (T)s;
+  l.x = (T)(c - (double)w.x);
+  l.y = (T)(s - (double)w.y);
+  return sizeof(T) == 4 ? c_mulw2<SIGN>(a, w, l) : c_mulw<SIGN>(a, w);
+}
 // a * (SIGN i)
 template <int SIGN, typename C>
 __device__ __forceinline__ C c_muli(C a) {
@@ -75,9 +113,6 @@ __device__ __forceinline__ void dft4(C& a0, C& a1, C& a2, C& a3) {
   }
 }
 
-template <typename C, typename T>
-__device__ __forceinline__ C c_const(T x, T y) { C r; r.x = x; r.y = y; return r; }
-
 template <int R, int SIGN, bool HALF, typename T, typename C>
 __device__ __forceinline__ void dft(C* v) {
   constexpr double h = 0.70710678118654752440;    // cos(pi/4)
@@ -94,8 +129,8 @@ __device__ __forceinline__ void dft(C* v) {
     dft4<SIGN, HALF>(v[0], v[2], v[4], v[6]);
     dft4<SIGN, HALF>(v[1], v[3], v[5], v[7]);
     const C o0 = v[1], o2 = c_muli<SIGN>(v[5]);
-    const C o1 = c_mulw<SIGN>(v[3], c_const<C, T>((T)h, -(T)h));
-    const C o3 = c_mulw<SIGN>(v[7], c_const<C, T>(-(T)h, -(T)h));
+    const C o1 = c_mulc<SIGN, T>(v[3], h, -h);
+    const C o3 = c_mulc<SIGN, T>(v[7], -h, -h);
     const C e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
     v[0] = c_add(e0, o0); v[4] = c_sub(e0, o0);
     v[1] = c_add(e1, o1); v[5] = c_sub(e1, o1);
@@ -105,15 +140,15 @@ __device__ __forceinline__ void dft(C* v) {
 #pragma unroll
     for (int n = 0; n < 4; n++) dft4<SIGN, HALF>(v[n], v[n + 4], v[n + 8], v[n + 12]);
     // element (n, k) at v[n + 4 k] times w16^(n k)
-    v[5] = c_mulw<SIGN>(v[5], c_const<C, T>((T)c1, -(T)s1));
-    v[9] = c_mulw<SIGN>(v[9], c_const<C, T>((T)h, -(T)h));
-    v[13] = c_mulw<SIGN>(v[13], c_const<C, T>((T)s1, -(T)c1));
-    v[6] = c_mulw<SIGN>(v[6], c_const<C, T>((T)h, -(T)h));
+    v[5] = c_mulc<SIGN, T>(v[5], c1, -s1);
+    v[9] = c_mulc<SIGN, T>(v[9], h, -h);
+    v[13] = c_mulc<SIGN, T>(v[13], s1, -c1);
+    v[6] = c_mulc<SIGN, T>(v[6], h, -h);
     v[10] = c_muli<SIGN>(v[10]);
-    v[14] = c_mulw<SIGN>(v[14], c_const<C, T>(-(T)h, -(T)h));
-    v[7] = c_mulw<SIGN>(v[7], c_const<C, T>((T)s1, -(T)c1));
-    v[11] = c_mulw<SIGN>(v[11], c_const<C, T>(-(T)h, -(T)h));
-    v[15] = c_mulw<SIGN>(v[15], c_const<C, T>(-(T)c1, (T)s1));
+    v[14] = c_mulc<SIGN, T>(v[14], -h, -h);
+    v[7] = c_mulc<SIGN, T>(v[7], s1, -c1);
+    v[11] = c_mulc<SIGN, T>(v[11], -h, -h);
+    v[15] = c_mulc<SIGN, T>(v[15], -c1, s1);
 #pragma unroll
     for (int k = 0; k < 4; k++) dft4<SIGN, false>(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     // X[k + 4 m] sits at v[4 k + m]: transpose
@@ -132,7 +167,8 @@ __device__ __forceinline__ void dft(C* v) {
 struct WarpSync { __device__ __forceinline__ void operator()() const { __syncwarp(); } };
 struct BlockSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
 
-template <typename T, int LOGN>
+// FINE: the twiddles with their second terms (FP32)
+template <typename T, int LOGN, bool FINE = false>
 struct Fft {
   typedef typename Cplx<T>::type C;
   static constexpr int N = 1 << LOGN;
@@ -156,8 +192,11 @@ struct Fft {
       for (int q = 0; q < SUB; q++) {
         const int m = (j + TPL * q) & (NS - 1);
 #pragma unroll
-        for (int e = 1; e < R; e++)
-          v[q * R + e] = c_mulw<SIGN>(v[q * R + e], tw[NS - E + (e - 1) * NS + m]);
+        for (int e = 1; e < R; e++) {
+          const int t = NS - E + (e - 1) * NS + m;
+          C& a = v[q * R + e];
+          a = FINE ? c_mulw2<SIGN>(a, tw[t], tw[N + t]) : c_mulw<SIGN>(a, tw[t]);
+        }
       }
     }
 #pragma unroll

@@ -96,7 +96,8 @@ inline PoissonMember poisson_member(const PoissonBuffers& b) {
   return m;
 }
 
-// twiddles of a transform of 2^logn points (complex T, at most 2^logn entries)
+// twiddles of a transform of 2^logn points (complex T, 2^logn entries in FP64,
+// 2^(logn + 1) with the second terms in FP32: 2^(logn + 4) bytes)
 template <typename T>
 int fft_twiddles(int logn, void* out);
 template <typename T>

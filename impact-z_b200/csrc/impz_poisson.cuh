@@ -86,8 +86,8 @@ __host__ __device__ constexpr int round_to(int v, int m) { return (v + m - 1) / 
 // slots (FP32), odd sixteen-byte slots (FP64).
 template <typename T, int LX, int LY>
 struct XyShape {
-  typedef Fft<T, LX> FX;
-  typedef Fft<T, LY> FY;
+  typedef Fft<T, LX, sizeof(T) == 4> FX;
+  typedef Fft<T, LY, sizeof(T) == 4> FY;
   typedef typename Cplx<T>::type C;
   static constexpr int nx = 1 << (LX - 1), ny = 1 << (LY - 1), hy = ny / 2;
   static constexpr int TA = round_to(hy * FX::TPL, 32), TB = round_to(nx * FY::TPL, 32);

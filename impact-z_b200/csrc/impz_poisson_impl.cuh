@@ -225,8 +225,8 @@ void unit_root(int logn, long long k, long double& re, long double& im) {
 }  // namespace
 
 // Twiddles of a transform of 2^logn points in the order the stages of
-// impz_fft.cuh read them; returns the number of entries written (at most
-// 2^logn).
+// impz_fft.cuh read them, and in FP32 what their rounding dropped from entry
+// 2^logn on; returns the number of entries, the second terms not counted.
 template <>
 int fft_twiddles<IMPZ_POISSON_T>(int logn, void* out) {
   typedef Cplx<IMPZ_POISSON_T>::type C;
@@ -242,6 +242,10 @@ int fft_twiddles<IMPZ_POISSON_T>(int logn, void* out) {
         unit_root(lns + lr, (long long)e * m, x, y);
         t[n].x = (IMPZ_POISSON_T)x;
         t[n].y = (IMPZ_POISSON_T)y;
+        if (sizeof(IMPZ_POISSON_T) == 4) {
+          t[(1 << logn) + n].x = (IMPZ_POISSON_T)(x - (long double)t[n].x);
+          t[(1 << logn) + n].y = (IMPZ_POISSON_T)(y - (long double)t[n].y);
+        }
       }
     lns += lr;
   }
