@@ -377,8 +377,9 @@ __device__ __forceinline__ void fft_z_conv_body(const PoissonDims& d, const Pois
 }
 
 // The three passes of a step took 70 us at 64x64x128 in FP32 as radix-2^3
-// groups in shared memory and take 35 so (FP64 97 and 56); at 64x64x2048,
-// where the spectrum (136 MB) no longer fits L2, 1498 and 393.
+// groups in shared memory and take 36 so (FP64 97 and 56); at 64x64x2048,
+// where the spectrum (136 MB) no longer fits L2, 1498 and 411 (35 and 394
+// without the second terms of the constants and of the x and y twiddles).
 template <typename T, int LZ>
 __global__ void __launch_bounds__((ZConv<T, LZ>::Z::NT))
     k_fft_z_conv(PoissonDims d, PoissonMember one, const PoissonMember* __restrict__ many) {
